@@ -9,6 +9,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -458,9 +459,11 @@ __global__ void k_colsum(int64_t rows, int cols, const float* __restrict__ dZ, f
     }
 }
 
-// Adam on the FP32 master weights; refresh the BF16 compute copy.
+#include "dtb_mlp_fused.cuh"
+
+// Adam on the FP32 master weights; refresh the BF16 compute copy (and the fused kernels' images of it).
 __global__ void k_adam(int64_t n, float* w, const float* __restrict__ g, float* m, float* v, __nv_bfloat16* wb,
-                       float lr, float b1, float b2, float eps, float c1, float c2)
+                       float lr, float b1, float b2, float eps, float c1, float c2, __nv_bfloat16* img, int in, int kx)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -471,13 +474,18 @@ __global__ void k_adam(int64_t n, float* w, const float* __restrict__ g, float* 
     v[i] = vi;
     const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     w[i] = wi;
-    wb[i] = __float2bfloat16_rn(wi);
+    const __nv_bfloat16 h = __float2bfloat16_rn(wi);
+    wb[i] = h;
+    if (img) net_write_img(i, in, kx, h, img);
 }
 
-__global__ void k_to_bf16(int64_t n, const float* __restrict__ w, __nv_bfloat16* wb)
+__global__ void k_to_bf16(int64_t n, const float* __restrict__ w, __nv_bfloat16* wb, __nv_bfloat16* img, int in, int kx)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) wb[i] = __float2bfloat16_rn(w[i]);
+    if (i >= n) return;
+    const __nv_bfloat16 h = __float2bfloat16_rn(w[i]);
+    wb[i] = h;
+    if (img) net_write_img(i, in, kx, h, img);
 }
 
 }  // namespace
@@ -489,12 +497,15 @@ struct dtb_mlp {
     int in = 0, H = 0;
     int64_t n_params = 0;
     int64_t o_W1, o_b1, o_W2, o_b2, o_W3, o_b3;
+    void* mem = nullptr;           // the allocation that holds everything up to the activations
     float* w = nullptr;            // FP32 master [n_params]
     __nv_bfloat16* wb = nullptr;   // BF16 compute copy
-    float* g = nullptr;            // gradients
+    __nv_bfloat16* img = nullptr;  // fused kernels: W2, W2^T and W1 as operand images (null: layer by layer)
+    int kx = 0;                    // ... padded inputs
+    float* g = nullptr;            // gradients, then the loss
     float* m = nullptr;            // Adam moments
     float* v = nullptr;
-    float* loss = nullptr;         // device scalar
+    float* loss = nullptr;         // device scalar: g[n_params]
     int64_t cap = 0;               // batch capacity of the activation buffers
     float *Z1 = nullptr, *H1 = nullptr, *Z2 = nullptr, *H2 = nullptr, *Y = nullptr;
     float *dY = nullptr, *dH2 = nullptr, *dZ2 = nullptr, *dH1 = nullptr, *dZ1 = nullptr;
@@ -583,6 +594,46 @@ int ensure_cap(dtb_mlp* p, int64_t B)
     return DTB_OK;
 }
 
+// hidden = 256, in <= 32: the whole pass in one kernel (target: also dZ2, dZ1 and the loss).
+int net_pass(dtb_mlp* p, const float* x, const float* target, int64_t B, float* y)
+{
+    NetArgs g;
+    std::memset(&g, 0, sizeof(g));
+    g.in = p->in; g.kx = p->kx; g.B = B;
+    g.x = x; g.target = target;
+    g.img2 = p->img; g.img2t = p->img + kNetImgW2; g.img1 = p->img + 2 * kNetImgW2;
+    g.b1 = p->w + p->o_b1; g.b2 = p->w + p->o_b2; g.b3 = p->w + p->o_b3;
+    g.w3 = p->wb + p->o_W3;
+    g.y = y; g.err = p->err;
+    const unsigned grid = cdiv(B, kNetRows);
+    if (!target) {
+        k_net<false><<<grid, kNetThreads, kNetSmem, p->stream>>>(g);
+    } else {
+        g.Z1 = p->Z1; g.H1 = p->H1; g.H2 = p->H2; g.dZ2 = p->dZ2; g.dZ1 = p->dZ1; g.dY = p->dY;
+        g.loss = p->loss;
+        k_net<true><<<grid, kNetThreads, kNetSmem, p->stream>>>(g);
+    }
+    MCK(cudaGetLastError());
+    return DTB_OK;
+}
+
+int net_gradient(dtb_mlp* p, const float* x, const float* target, int64_t B)
+{
+    MCK(cudaMemsetAsync(p->g, 0, sizeof(float) * (size_t)(p->n_params + 1), p->stream));   // and the loss
+    if (int rc = net_pass(p, x, target, B, nullptr)) return rc;
+    GradArgs a;
+    a.in = p->in; a.kx = p->kx; a.B = B;
+    // one split of rows per SM pair (two halves of the output rows each), whole stages
+    a.rows_per_split = ((B + 73) / 74 + kGradStage - 1) / kGradStage * kGradStage;
+    a.x = x; a.H1 = p->H1; a.H2 = p->H2; a.dZ2 = p->dZ2; a.dZ1 = p->dZ1; a.dY = p->dY;
+    a.gW1 = p->g + p->o_W1; a.gb1 = p->g + p->o_b1; a.gW2 = p->g + p->o_W2; a.gb2 = p->g + p->o_b2;
+    a.gW3 = p->g + p->o_W3; a.gb3 = p->g + p->o_b3;
+    a.err = p->err;
+    k_net_grad<<<dim3(2, cdiv(B, a.rows_per_split)), kNetThreads, kGradSmem, p->stream>>>(a);
+    MCK(cudaGetLastError());
+    return DTB_OK;
+}
+
 int forward(dtb_mlp* p, const float* x, int64_t B, float* y)
 {
     const int in = p->in, H = p->H;
@@ -659,19 +710,36 @@ int dtb_mlp_create(int in_dim, int hidden, uint64_t seed, int device, dtb_mlp** 
     for (int64_t i = 0; i < (int64_t)hidden * in_dim; ++i) w[(size_t)(p->o_W1 + i)] = (2.0f * uni() - 1.0f) * a1;
     for (int64_t i = 0; i < (int64_t)hidden * hidden; ++i) w[(size_t)(p->o_W2 + i)] = (2.0f * uni() - 1.0f) * a2;
     for (int64_t i = 0; i < hidden; ++i) w[(size_t)(p->o_W3 + i)] = (2.0f * uni() - 1.0f) * a2;
-    cudaError_t e = cudaMalloc(&p->w, sizeof(float) * (size_t)o);
-    if (e == cudaSuccess) e = cudaMalloc(&p->wb, sizeof(__nv_bfloat16) * (size_t)o);
-    if (e == cudaSuccess) e = cudaMalloc(&p->g, sizeof(float) * (size_t)o);
-    if (e == cudaSuccess) e = cudaMalloc(&p->m, sizeof(float) * (size_t)o);
-    if (e == cudaSuccess) e = cudaMalloc(&p->v, sizeof(float) * (size_t)o);
-    if (e == cudaSuccess) e = cudaMalloc(&p->loss, sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&p->err, sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(p->err, 0, sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemcpy(p->w, w.data(), sizeof(float) * (size_t)o, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(p->m, 0, sizeof(float) * (size_t)o);
-    if (e == cudaSuccess) e = cudaMemset(p->v, 0, sizeof(float) * (size_t)o);
+    // one allocation: masters, gradients and loss, moments, BF16 copy, operand images, error flag
+    const bool fused = hidden == kNetH && in_dim <= kNetMaxIn;
+    const size_t f4 = (sizeof(float) * (size_t)(o + 1) + 255) & ~(size_t)255;
+    const size_t f2 = (sizeof(__nv_bfloat16) * (size_t)o + 255) & ~(size_t)255;
+    const size_t fi = fused ? sizeof(__nv_bfloat16) * (size_t)(2 * kNetImgW2 + kNetH * kNetMaxIn) : 0;
+    char* mem = nullptr;
+    cudaError_t e = cudaMalloc(&mem, 4 * f4 + f2 + fi + 256);
     if (e == cudaSuccess) {
-        k_to_bf16<<<cdiv(o, 256), 256>>>(o, p->w, p->wb);
+        p->mem = mem;
+        p->w = (float*)mem; p->g = (float*)(mem + f4); p->m = (float*)(mem + 2 * f4); p->v = (float*)(mem + 3 * f4);
+        p->loss = p->g + o;
+        p->wb = (__nv_bfloat16*)(mem + 4 * f4);
+        p->err = (unsigned*)(mem + 4 * f4 + f2 + fi);
+        if (fused) {
+            p->kx = in_dim <= 16 ? 16 : 32;
+            p->img = (__nv_bfloat16*)(mem + 4 * f4 + f2);
+        }
+        // zero moments, error flag and the padded inputs' weights
+        e = cudaMemset(mem + f4, 0, 3 * f4 + f2 + fi + 256);
+    }
+    static std::atomic<uint64_t> ready{0};   // devices whose attributes are set
+    if (e == cudaSuccess && fused && !((ready.load() >> (device & 63)) & 1)) {
+        e = cudaFuncSetAttribute(k_net<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNetSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_net<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNetSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_net_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem);
+        if (e == cudaSuccess) ready.fetch_or(1ull << (device & 63));
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(p->w, w.data(), sizeof(float) * (size_t)o, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_to_bf16<<<cdiv(o, 256), 256>>>(o, p->w, p->wb, p->img, in_dim, p->kx);
         e = cudaDeviceSynchronize();
     }
     if (prev >= 0) cudaSetDevice(prev);
@@ -689,7 +757,7 @@ int dtb_mlp_destroy(dtb_mlp* p)
     int prev = -1;
     cudaGetDevice(&prev);
     cudaSetDevice(p->device);
-    void* bufs[] = {p->w, p->wb, p->g, p->m, p->v, p->loss, p->err, p->Z1, p->H1, p->Z2, p->H2, p->Y,
+    void* bufs[] = {p->mem, p->Z1, p->H1, p->Z2, p->H2, p->Y,
                     p->dY, p->dH2, p->dZ2, p->dH1, p->dZ1};
     for (void* b : bufs) if (b) cudaFree(b);
     if (prev >= 0) cudaSetDevice(prev);
@@ -725,7 +793,7 @@ int dtb_mlp_set_params(dtb_mlp* p, const float* src, int where)
     if (!p || !src) return mlp_fail(DTB_ERR_ARG, "null argument");
     MCK(cudaMemcpyAsync(p->w, src, sizeof(float) * (size_t)p->n_params,
                         where == DTB_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, p->stream));
-    k_to_bf16<<<cdiv(p->n_params, 256), 256, 0, p->stream>>>(p->n_params, p->w, p->wb);
+    k_to_bf16<<<cdiv(p->n_params, 256), 256, 0, p->stream>>>(p->n_params, p->w, p->wb, p->img, p->in, p->kx);
     MCK(cudaGetLastError());
     MCK(cudaStreamSynchronize(p->stream));
     return DTB_OK;
@@ -734,6 +802,7 @@ int dtb_mlp_set_params(dtb_mlp* p, const float* src, int where)
 int dtb_mlp_forward(dtb_mlp* p, const float* x, int64_t B, float* y)
 {
     if (!p || !x || !y || B < 1) return mlp_fail(DTB_ERR_ARG, "bad argument");
+    if (p->img) return net_pass(p, x, nullptr, B, y);
     if (int rc = ensure_cap(p, B)) return rc;
     return forward(p, x, B, y);
 }
@@ -742,8 +811,12 @@ int dtb_mlp_gradient(dtb_mlp* p, const float* x, const float* target, int64_t B,
 {
     if (!p || !x || !target || B < 1) return mlp_fail(DTB_ERR_ARG, "bad argument");
     if (int rc = ensure_cap(p, B)) return rc;
-    if (int rc = forward(p, x, B, p->Y)) return rc;
-    if (int rc = backward(p, x, target, B)) return rc;
+    if (p->img) {
+        if (int rc = net_gradient(p, x, target, B)) return rc;
+    } else {
+        if (int rc = forward(p, x, B, p->Y)) return rc;
+        if (int rc = backward(p, x, target, B)) return rc;
+    }
     if (grad) MCK(cudaMemcpyAsync(grad, p->g, sizeof(float) * (size_t)p->n_params, cudaMemcpyDeviceToDevice, p->stream));
     if (loss) MCK(cudaMemcpyAsync(loss, p->loss, sizeof(float), cudaMemcpyDeviceToDevice, p->stream));
     return DTB_OK;
@@ -756,7 +829,7 @@ int dtb_mlp_train_step(dtb_mlp* p, const float* x, const float* target, int64_t 
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f - std::pow(b1, (float)p->t), c2 = 1.0f - std::pow(b2, (float)p->t);
     k_adam<<<cdiv(p->n_params, 256), 256, 0, p->stream>>>(p->n_params, p->w, p->g, p->m, p->v, p->wb, lr, b1, b2,
-                                                          1e-8f, c1, c2);
+                                                          1e-8f, c1, c2, p->img, p->in, p->kx);
     MCK(cudaGetLastError());
     return DTB_OK;
 }

@@ -50,3 +50,18 @@ def test_rate_surrogate_learns_rate_map():
     err_net = np.sqrt(np.mean((pred - target) ** 2))
     err_persist = np.sqrt(np.mean((hist[:, -1] - target) ** 2))
     assert err_net < 0.25 * err_persist, (err_net, err_persist)
+
+
+@pytest.mark.parametrize("inputs,hidden", [(1, 256), (16, 256), (17, 256), (32, 256), (33, 256), (14, 64)])
+@pytest.mark.parametrize("B", [64, 128, 129, 4801])
+def test_shapes_match_oracle(inputs, hidden, B):
+    """Whole and partial row tiles, the input paddings, and sizes the fused kernels do not take."""
+    rng = np.random.default_rng([B, inputs])
+    m = MLP(inputs, hidden, seed=5, device=0)
+    x = rng.normal(0, 1, (B, inputs)).astype(np.float32)
+    t = rng.normal(0, 1, B).astype(np.float32)
+    y_ref, loss_ref, g_ref = mlp_oracle.forward_backward(m.params(), x, t, inputs, hidden)
+    np.testing.assert_allclose(m.forward(torch.from_numpy(x)).cpu().numpy(), y_ref, rtol=1e-4, atol=1e-5)
+    g, loss = m.gradient(torch.from_numpy(x), torch.from_numpy(t))
+    assert abs(loss - loss_ref) <= 1e-4 * loss_ref
+    assert np.abs(g.cpu().numpy() - g_ref).max() <= 1e-4 * np.abs(g_ref).max()
