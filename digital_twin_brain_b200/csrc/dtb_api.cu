@@ -1135,6 +1135,22 @@ static BoldScalars<T> bold_scalars(const dtb_bold* m)
     return c;
 }
 
+static BoldConst bold_const(double eps, double ts, double tf, double t0, double alpha, double E0, double dt)
+{
+    BoldConst c;
+    c.eps = eps; c.r_ts = 1.0 / ts; c.r_tf = 1.0 / tf; c.r_t0 = 1.0 / t0; c.r_E0 = 1.0 / E0; c.dt = dt;
+    c.base = 1.0 - E0;
+    c.exv = 1.0 / alpha;
+    c.l_hi = c.l_lo = 0.0;
+    c.fast = (c.exv == 5.0 && c.base > 0.0 && c.base < 1.0) ? 1 : 0;
+    if (c.fast) {
+        const long double l = logl((long double)c.base);
+        c.l_hi = (double)l;
+        c.l_lo = (double)(l - (long double)c.l_hi);
+    }
+    return c;
+}
+
 // ------------------------------------------------------------ C ABI
 extern "C" {
 
@@ -2629,9 +2645,10 @@ int dtb_bold_run_steps(dtb_bold* m, const void* u, int n_steps, double u_floor, 
                                                            (float*)m->s, (float*)m->q, (float*)m->v, (float*)m->f,
                                                            (float*)dout, bold_scalars<float>(m));
     else
-        k_bold_run_steps<double><<<gr, 128, 0, m->stream>>>(m->R, (const double*)du, n_steps, u_floor,
-                                                            (double*)m->s, (double*)m->q, (double*)m->v,
-                                                            (double*)m->f, (double*)dout, bold_scalars<double>(m));
+        k_bold_run_steps_f64<<<grid_for(m->R, kBoldThreads), kBoldThreads, 0, m->stream>>>(
+            m->R, (const double*)du, n_steps, u_floor, (double*)m->s, (double*)m->q, (double*)m->v, (double*)m->f,
+            (double*)dout, bold_const(m->eps, m->ts, m->tf, m->t0, m->alpha, m->E0, m->dt), 7.0 * m->E0,
+            2.0 * m->E0 - 0.2, m->V0);
     CK(cudaGetLastError());
     if (where == DTB_HOST) {
         CK(cudaMemcpyAsync(out, m->tmp_o, bytes, cudaMemcpyDeviceToHost, m->stream));
@@ -2722,8 +2739,8 @@ int dtb_block_attach_bold(dtb_block* b, int n_regions, const int32_t* sub_to_reg
     bd.region_n = drn;
     bd.s = st; bd.q = st + n_regions; bd.v = st + 2 * n_regions; bd.f = st + 3 * n_regions;
     bd.act = st + 4 * n_regions; bd.out = st + 5 * n_regions;
-    bd.epsilon = epsilon; bd.tao_s = tao_s; bd.tao_f = tao_f; bd.tao_0 = tao_0; bd.div_alpha = 1.0 / alpha;
-    bd.E0 = E_0; bd.V0 = V_0; bd.delta_t = delta_t;
+    bd.c = bold_const(epsilon, tao_s, tao_f, tao_0, alpha, E_0, delta_t);
+    bd.E0 = E_0; bd.V0 = V_0;
     b->bold_R = n_regions;
     RET(rebuild_groups(b, sub_to_region));
     for (auto& ge : b->graph) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }

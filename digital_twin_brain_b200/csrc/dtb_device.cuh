@@ -81,12 +81,22 @@ struct RunParams {
 };
 static_assert(sizeof(RunParams) == 16, "RunParams layout");
 
+// Constants of the float64 BOLD step (bold_model_pytorch.py:43-78): reciprocals of the time
+// constants and of E_0, and ln(1 - E_0) in two parts.
+struct BoldConst {
+    double eps, r_ts, r_tf, r_t0, r_E0, dt;
+    double base, l_hi, l_lo;   // 1 - E_0 and its logarithm
+    double exv;                // 1 / alpha
+    int fast;                  // 1: 1 / alpha is 5 and 0 < base < 1 (the model's own constants)
+};
+
 struct BoldDev {
+    BoldConst c;
     int n_regions;               // 0: no BOLD attached
     const int32_t* sub_region;   // [n_sub] -> region or -1
     const double* region_n;      // [R] neurons in region
     double* s; double* q; double* v; double* f; double* act; double* out;   // [R]
-    double epsilon, tao_s, tao_f, tao_0, div_alpha, E0, V0, delta_t;
+    double E0, V0;
 };
 
 struct DevState {
