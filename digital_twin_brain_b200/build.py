@@ -21,7 +21,7 @@ PROBE_LIB = os.path.join(PKG, "libdtb_bench_probe.so")
 PROBE_SOURCES = ["bench_probe.cu"]
 
 SOURCES = ["dtb_api.cu", "dtb_prealloc.cu", "dtb_mlp.cu", "dtb_io.cpp"]
-HEADERS = ["dtb_device.cuh", "dtb_kernels.cuh", "dtb_mlp_fused.cuh", "dtb_io.h"]
+HEADERS = ["dtb_device.cuh", "dtb_kernels.cuh", "dtb_small.cuh", "dtb_mlp_fused.cuh", "dtb_io.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -19,6 +19,7 @@
 #include "dtb.h"
 #include "dtb_io.h"
 #include "dtb_kernels.cuh"
+#include "dtb_small.cuh"
 
 using namespace dtb;
 
@@ -184,6 +185,14 @@ struct dtb_block {
     cudaGraphExec_t graph[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     int graph_len[7] = {0, 0, 0, 0, 0, 0, 0};
     bool use_graphs = true;
+    // small-network step loop (k_small): second-parity accumulators
+    uint32_t* d_spk2 = nullptr;
+    uint32_t* d_nact2 = nullptr;
+    double* d_vsum2 = nullptr;
+    uint32_t* d_unmapped2 = nullptr;
+    int grp_n_sub = -1;           // subblocks when the statistics groups were built
+    bool knobs_set = false;       // the caller chose a schedule (dtb_block_set_tuning): launch per step as asked
+    bool chunk_set = false;
     // attached BOLD
     int bold_R = 0;
     // gamma-distributed g_ui (per-neuron factors; ds.gnrn points here while active)
@@ -354,6 +363,8 @@ static int alloc_state(dtb_block* b)
     RET(dalloc(b, &s.ctl, 1));
     RET(dalloc(b, &s.ev_part, kEvParts));
     RET(dalloc(b, &s.unmapped_nact, 1));
+    RET(dalloc(b, &b->d_unmapped2, 1));
+    CK(cudaMemsetAsync(b->d_unmapped2, 0, sizeof(uint32_t), b->stream));
     RET(dalloc(b, &b->d_err, 4));
     CK(cudaMemsetAsync(s.J2, 0, sizeof(float2) * 2 * (size_t)jps, b->stream));
     CK(cudaMemsetAsync(s.tlast, 0, sizeof(float) * (size_t)N, b->stream));
@@ -390,6 +401,12 @@ static int upload_class_tables(dtb_block* b)
         RET(dalloc(b, &s.sub_nact, (size_t)cap));
         RET(dalloc(b, &s.sub_vsum, (size_t)cap));
         RET(dalloc(b, &s.win_spk, (size_t)cap));
+        RET(dalloc(b, &b->d_spk2, (size_t)cap));
+        RET(dalloc(b, &b->d_nact2, (size_t)cap));
+        RET(dalloc(b, &b->d_vsum2, (size_t)cap));
+        CK(cudaMemsetAsync(b->d_spk2, 0, sizeof(uint32_t) * cap, b->stream));
+        CK(cudaMemsetAsync(b->d_nact2, 0, sizeof(uint32_t) * cap, b->stream));
+        CK(cudaMemsetAsync(b->d_vsum2, 0, sizeof(double) * cap, b->stream));
         CK(cudaMemsetAsync(s.win_spk, 0, sizeof(unsigned long long) * cap, b->stream));
         CK(cudaMemsetAsync(s.sub_spk, 0, sizeof(uint32_t) * cap, b->stream));
         CK(cudaMemsetAsync(s.sub_nact, 0, sizeof(uint32_t) * cap, b->stream));
@@ -542,15 +559,15 @@ static int finish_create(dtb_block* b)
 }
 
 // ------------------------------------------------------------ launches
-// Statistics outside the update kernel when the subblock / region count is
-// large: groups = BOLD regions with their subblocks, plus lone subblocks.
+// Statistics groups = BOLD regions with their subblocks, plus lone subblocks: the
+// small-network step loop folds statistics by group, and so does k_stats outside the
+// update kernel when the subblock / region count is large.
 static int rebuild_groups(dtb_block* b, const int32_t* sub_to_region)
 {
     DevState& s = b->ds;
     const int n_sub = b->n_sub;
     const int R = b->bold_R;
     s.stats_ext = (n_sub > 512 || R > 128) ? 1 : 0;
-    if (!s.stats_ext) return DTB_OK;
     std::vector<int32_t> ptr, sub, reg;
     if (R > 0 && sub_to_region) {
         std::vector<std::vector<int32_t>> members((size_t)R);
@@ -570,6 +587,8 @@ static int rebuild_groups(dtb_block* b, const int32_t* sub_to_region)
         for (int i = 0; i <= n_sub; ++i) ptr.push_back(i);
         for (int i = 0; i < n_sub; ++i) { sub.push_back(i); reg.push_back(-1); }
     }
+    CK(cudaStreamSynchronize(b->stream));   // the previous tables are no longer in use
+    dfree(b, s.grp_ptr); dfree(b, s.grp_sub); dfree(b, s.grp_region);
     int32_t *dp = nullptr, *ds = nullptr, *dr = nullptr;
     RET(dalloc(b, &dp, ptr.size()));
     RET(dalloc(b, &ds, std::max<size_t>(1, sub.size())));
@@ -579,6 +598,7 @@ static int rebuild_groups(dtb_block* b, const int32_t* sub_to_region)
     if (!reg.empty()) CK(cudaMemcpy(dr, reg.data(), sizeof(int32_t) * reg.size(), cudaMemcpyHostToDevice));
     s.grp_ptr = dp; s.grp_sub = ds; s.grp_region = dr;
     s.n_groups = (int)reg.size();
+    b->grp_n_sub = n_sub;
     return DTB_OK;
 }
 
@@ -1078,6 +1098,20 @@ static int set_run_params(dtb_block* b, float noise_rate, int isolated)
     return DTB_OK;
 }
 
+// The device's error flags, reported once: they are cleared.
+static int report_err(dtb_block* b, uint32_t err)
+{
+    if (!err) return DTB_OK;
+    CK(cudaMemsetAsync(&b->ds.ctl->err, 0, sizeof(uint32_t), b->stream));
+    CK(cudaStreamSynchronize(b->stream));
+    if (err & kErrGeneralSkipped)
+        return fail(DTB_ERR_STATE, "internal: an update ran without the I_syn override or gamma g_ui it needed");
+    if (err & (kErrStageTimeout | kErrStageDrain))
+        return fail(DTB_ERR_CUDA, "a staged state copy did not complete in time%s (the update loaded that "
+                    "state from global memory instead)", (err & kErrStageDrain) ? " and had not landed at exit" : "");
+    return DTB_OK;
+}
+
 // Copies `rows` stats rows to the caller (row offset `row0` of the outputs).
 static int emit_stats(dtb_block* b, int rows, int64_t row0, float* sum_out, float* mean_out, uint32_t* nact_out,
                       int where, std::vector<uint32_t>* nact_host)
@@ -1102,15 +1136,7 @@ static int emit_stats(dtb_block* b, int rows, int64_t row0, float* sum_out, floa
         uint32_t* herr = reinterpret_cast<uint32_t*>(p + ((2 * bs + bn + 7) & ~(size_t)7));
         CK(cudaMemcpyAsync(herr, &b->ds.ctl->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream));
         CK(cudaStreamSynchronize(b->stream));
-        if (*herr) {   // reported once: the flags are cleared
-            CK(cudaMemsetAsync(&b->ds.ctl->err, 0, sizeof(uint32_t), b->stream));
-            CK(cudaStreamSynchronize(b->stream));
-            if (*herr & kErrGeneralSkipped)
-                return fail(DTB_ERR_STATE, "internal: an update ran without the I_syn override or gamma g_ui it needed");
-            if (*herr & (kErrStageTimeout | kErrStageDrain))
-                return fail(DTB_ERR_CUDA, "a staged state copy did not complete in time%s (the update loaded that "
-                            "state from global memory instead)", (*herr & kErrStageDrain) ? " and had not landed at exit" : "");
-        }
+        RET(report_err(b, *herr));
         if (where == DTB_HOST) {
             if (sum_out && bs) std::memcpy(sum_out + row0 * ns, p, bs);
             if (mean_out && bs) std::memcpy(mean_out + row0 * ns, p + bs, bs);
@@ -1121,6 +1147,94 @@ static int emit_stats(dtb_block* b, int rows, int64_t row0, float* sum_out, floa
             std::memcpy(nact_host->data(), p + 2 * bs, bn);
         }
     }
+    return DTB_OK;
+}
+
+// CTAs of the small-network step loop (k_small) for a run of method `method`, or 0 when the
+// per-step kernels serve it.
+static int small_ctas(const dtb_block* b, int method)
+{
+    const DevState& s = b->ds;
+    if (b->N <= 0 || b->N > kSmallMaxNeurons) return 0;
+    if (method != DTB_MODE_PUSH && method != kModeSlots) return 0;
+    if (method == kModeSlots && b->pull_method != 0) return 0;           // the caller asked for the slot kernels
+    if (b->knobs_set || !b->use_graphs) return 0;
+    if (!b->has_pull || !b->has_push || !b->has_qpos) return 0;
+    if (b->override_live || s.gnrn || s.n_src > 0 || s.forced_active) return 0;   // the general update
+    if (!staged_layout(s) || !s.tile_cls || b->grp_n_sub != b->n_sub) return 0;
+    if (b->S > 0x7fffffffLL) return 0;                                   // 32-bit synapse offsets
+    const int nt = (int)((b->N + kWarpNeurons - 1) / kWarpNeurons);
+    int ctas = (nt + kSmallTilesFew - 1) / kSmallTilesFew;
+    return ctas < kSmallClusterMax ? ctas : kSmallClusterMax;
+}
+
+// n steps of k_small and their statistics (rows row0.. of the outputs).  Device outputs are written
+// by the kernel itself; small host outputs go to pinned memory the same way, so that a call costs
+// one launch and one synchronisation.  nact_host: the propagated counts on the host (nullable).
+constexpr int64_t kSmallHostValues = 8192;   // statistics values written to pinned memory by the kernel
+
+static int run_small(dtb_block* b, int ctas, int n, float noise_rate, int isolated, int64_t row0, float* sum_out,
+                     float* mean_out, uint32_t* nact_out, int where, std::vector<uint32_t>* nact_host)
+{
+    static std::atomic<uint64_t> ready{0};                               // devices whose attribute is set
+    const uint64_t bit = 1ull << (b->device & 63);
+    if (!(ready.load() & bit)) {
+        CK(cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax));
+        ready.fetch_or(bit);
+    }
+    const int nt = (int)((b->N + kWarpNeurons - 1) / kWarpNeurons);
+    SmallArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.n_steps = n;
+    a.tiles_per_cta = (nt + ctas - 1) / ctas;
+    a.cap = (uint32_t)small_cap(a.tiles_per_cta);
+    a.tile_magic = (65536u + (uint32_t)a.tiles_per_cta - 1u) / (uint32_t)a.tiles_per_cta;   // exact for tile < 96 (tested)
+    a.isolated = isolated ? 1 : 0;
+    a.noise_rate = noise_rate;
+    a.write_v = b->ds.n_samples > 0 ? 1 : 0;
+    a.spk0 = b->ds.sub_spk;   a.spk1 = b->d_spk2;
+    a.nact0 = b->ds.sub_nact; a.nact1 = b->d_nact2;
+    a.vsum0 = b->ds.sub_vsum; a.vsum1 = b->d_vsum2;
+    a.unmapped0 = b->ds.unmapped_nact; a.unmapped1 = b->d_unmapped2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = small_smem(a.tiles_per_cta, (int)a.cap);
+    cfg.stream = b->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    DevState s = b->ds;
+    const size_t ns = (size_t)b->n_sub, nv = (size_t)n * ns;
+    const bool pinned = (where == DTB_HOST && (int64_t)nv <= kSmallHostValues) || (where == DTB_DEVICE && nact_host);
+    float* ph = nullptr;
+    if (pinned) {
+        RET(ensure_pinned(b, 2 * nv * sizeof(float) + ((size_t)n + 1) * sizeof(uint32_t)));
+        ph = reinterpret_cast<float*>(b->pinned);
+        a.host_nact = reinterpret_cast<uint32_t*>(ph + 2 * nv);
+    }
+    if (where == DTB_DEVICE) {
+        if (sum_out) s.st_spk = sum_out + (size_t)row0 * ns;
+        if (mean_out) s.st_mean = mean_out + (size_t)row0 * ns;
+        if (nact_out) s.st_nact = nact_out + row0;
+    } else if (pinned) {
+        s.st_spk = ph;
+        s.st_mean = ph + nv;
+    }
+    CK(cudaLaunchKernelEx(&cfg, k_small, s, a));
+    b->launches++;
+    if (!pinned) return where == DTB_HOST ? emit_stats(b, n, row0, sum_out, mean_out, nact_out, where, nact_host) : DTB_OK;
+    CK(cudaStreamSynchronize(b->stream));
+    RET(report_err(b, a.host_nact[n]));
+    if (where == DTB_HOST) {
+        if (sum_out && nv) std::memcpy(sum_out + (size_t)row0 * ns, ph, nv * sizeof(float));
+        if (mean_out && nv) std::memcpy(mean_out + (size_t)row0 * ns, ph + nv, nv * sizeof(float));
+        if (nact_out) std::memcpy(nact_out + row0, a.host_nact, sizeof(uint32_t) * (size_t)n);
+    }
+    if (nact_host) nact_host->assign(a.host_nact, a.host_nact + n);
     return DTB_OK;
 }
 
@@ -1740,15 +1854,30 @@ int dtb_block_run(dtb_block* b, int n_steps, float noise_rate, int isolated, int
     while (done < n_steps) {
         const int m = choose_mode(b, mode);
         const int mm = resolve_method(b, m);
-        RET(ensure_method(b, mm));
         const uint32_t cap = b->stats_cap;
-        int n = (int)std::min<int64_t>(n_steps - done, (int64_t)std::min<uint32_t>(cap, (uint32_t)b->chunk));
-        RET(set_run_params(b, noise_rate, isolated));
-        RET(enqueue_chunk(b, n, mm));
-        b->steps += (uint64_t)n;
+        const int small = small_ctas(b, mm);
+        if (!small) RET(ensure_method(b, mm));
+        int n;
+        if (small > 0) {
+            // one launch takes the steps; DTB_MODE_AUTO still reconsiders the method every chunk
+            const uint32_t per = (mode == DTB_MODE_AUTO || b->chunk_set) ? (uint32_t)b->chunk : kSmallSteps;
+            n = (int)std::min<int64_t>(n_steps - done, (int64_t)std::min<uint32_t>(cap, per));
+            RET(flush_bins(b));
+        } else {
+            n = (int)std::min<int64_t>(n_steps - done, (int64_t)std::min<uint32_t>(cap, (uint32_t)b->chunk));
+        }
         std::vector<uint32_t> nact;
         const bool want_nact = (mode == DTB_MODE_AUTO) || (m == DTB_MODE_PULL && b->has_qpos && b->pull_method == 0);
-        RET(emit_stats(b, n, done, sum_out, mean_out, nact_out, where, want_nact ? &nact : nullptr));
+        if (small > 0) {
+            b->steps += (uint64_t)n;
+            RET(run_small(b, small, n, noise_rate, isolated, done, sum_out, mean_out, nact_out, where,
+                          want_nact ? &nact : nullptr));
+        } else {
+            RET(set_run_params(b, noise_rate, isolated));
+            RET(enqueue_chunk(b, n, mm));
+            b->steps += (uint64_t)n;
+            RET(emit_stats(b, n, done, sum_out, mean_out, nact_out, where, want_nact ? &nact : nullptr));
+        }
         if (want_nact && n > 0) {
             double tot = 0.0;
             for (uint32_t v : nact) tot += v;
@@ -1915,6 +2044,10 @@ int dtb_block_set_tuning(dtb_block* b, int key, int64_t value)
     }
     default: return fail(DTB_ERR_ARG, "unknown tuning key %d", key);
     }
+    if (key == DTB_TUNE_CHUNK) b->chunk_set = true;
+    else if (key != DTB_TUNE_PULL_THRESHOLD_PPM && key != DTB_TUNE_PULL_METHOD && key != DTB_TUNE_PUSH_METHOD &&
+             key != DTB_TUNE_USE_GRAPHS)
+        b->knobs_set = true;
     drop_graphs(b);
     return DTB_OK;
 }
