@@ -166,7 +166,7 @@ struct dtb_block {
     double last_frac = -1.0;
     double pull_threshold = 0.05;
     int chunk = 32;
-    int scatter_wpw = 32;         // bitmask words per warp in the push scatter
+    int scatter_wpw = 0;          // bitmask words per warp in the push scatter (0: by network size)
     int scatter_variant = 0;      // 0: registers unbounded, 1: budgeted for 6 resident CTAs per SM
     int step_variant = 3;         // 0: 2 resident CTAs/SM register budget, 1: 3; 2..4: staged, 2..4 CTAs/SM
     // ordered push (bit-exact pull through per-neuron slots)
@@ -769,9 +769,12 @@ static int launch_src(dtb_block* b, const DevState& s)
 }
 
 // gather: 0 none, kGatherRows (fused pull gather), kGatherSlots / kGatherMasks (ordered push)
-static int launch_update(dtb_block* b, const DevState& s, int gather, bool forced)
+// defer: a scatter launched with the same flag follows and folds the step's statistics.
+static int launch_update(dtb_block* b, const DevState& s_in, int gather, bool forced, bool defer = false)
 {
-    if (s.N <= 0) return DTB_OK;
+    if (s_in.N <= 0) return DTB_OK;
+    DevState s = s_in;
+    s.defer = defer ? 1 : 0;
     if (s.n_src > 0 && s.forced_active == s.src_val) {   // input neurons replay their raster
         RET(launch_src(b, s));
         forced = true;
@@ -796,8 +799,12 @@ static int launch_update(dtb_block* b, const DevState& s, int gather, bool force
     }
     CK(cudaGetLastError());
     b->launches++;
-    return launch_stats(b, s);
+    return defer ? DTB_OK : launch_stats(b, s);
 }
+
+// A scatter follows every update of these runs: its first CTAs can fold the statistics (sampled
+// neurons are read right after the update, so they keep the folding there).
+static bool can_defer(const dtb_block* b) { return b->ds.n_samples == 0 && b->ds.N > 0 && b->grp_n_sub == b->n_sub; }
 
 // Folds the propagation of the last step into J (end of a pull run).
 static int launch_gather_only(dtb_block* b, const DevState& s, int gather = kGatherRows)
@@ -812,18 +819,30 @@ static int launch_gather_only(dtb_block* b, const DevState& s, int gather = kGat
     return DTB_OK;
 }
 
-// how: kScatterJ (push), kScatterSlots / kScatterMasks (ordered push)
-static int launch_scatter(dtb_block* b, const DevState& s, int how = kScatterJ)
+// Bitmask words per warp: the caller's, or enough warps for every SM (a step's few firing rows
+// should not queue behind each other) and at most four words, past which a warp's rows serialise.
+// Measured, N = 31,013: 1 / 4 / 32 words 9.0 / 10.8 / 16.3 us; 1e6: 25.2 / 19.9 / 27.2; 1.2e7:
+// 226 / 196 / 243 (the row-list kernel).
+static int scatter_words(const dtb_block* b)
 {
-    const int wpw = b->scatter_wpw;
+    if (b->scatter_wpw > 0) return b->scatter_wpw;
+    int w = 1;
+    while (w < 4 && b->ds.n_words >= (int64_t)8192 * w) w *= 2;
+    return w;
+}
+
+// how: kScatterJ (push), kScatterSlots / kScatterMasks (ordered push)
+static int launch_scatter(dtb_block* b, const DevState& s, int how = kScatterJ, bool defer = false)
+{
+    const int wpw = scatter_words(b);
     const int64_t warps = (s.n_words + wpw - 1) / wpw;
-    const unsigned grid = grid_for(warps * 32, kScatterThreads);
+    const int stat = defer ? std::max(1, (int)grid_for(s.n_groups, kStatThreads)) : 0;
+    const unsigned grid = grid_for(warps * 32, kScatterThreads) + (unsigned)stat;
     if (grid == 0) return DTB_OK;
-    const size_t smem = sizeof(uint32_t) * 32 * (size_t)wpw * (kScatterThreads / 32);   // <= 32 KB
-    if (how == kScatterSlots) k_scatter<kScatterSlots><<<grid, kScatterThreads, smem, b->stream>>>(s, wpw);
-    else if (how == kScatterMasks) k_scatter<kScatterMasks><<<grid, kScatterThreads, smem, b->stream>>>(s, wpw);
-    else if (b->scatter_variant == 1) k_scatter<kScatterJ, 6><<<grid, kScatterThreads, smem, b->stream>>>(s, wpw);
-    else k_scatter<kScatterJ><<<grid, kScatterThreads, smem, b->stream>>>(s, wpw);
+    if (how == kScatterSlots) k_scatter<kScatterSlots><<<grid, kScatterThreads, 0, b->stream>>>(s, wpw, stat);
+    else if (how == kScatterMasks) k_scatter<kScatterMasks><<<grid, kScatterThreads, 0, b->stream>>>(s, wpw, stat);
+    else if (b->scatter_variant == 1) k_scatter<kScatterJ, 6><<<grid, kScatterThreads, 0, b->stream>>>(s, wpw, stat);
+    else k_scatter<kScatterJ, 4><<<grid, kScatterThreads, 0, b->stream>>>(s, wpw, stat);
     CK(cudaGetLastError());
     b->launches++;
     return DTB_OK;
@@ -991,10 +1010,11 @@ static int enqueue_steps(dtb_block* b, int n, int mode)
 {
     if (n <= 0) return DTB_OK;
     const DevState& s = b->ds;
+    const bool defer = can_defer(b);
     if (mode == DTB_MODE_PUSH) {
         for (int k = 0; k < n; ++k) {
-            RET(launch_update(b, s, 0, false));
-            RET(launch_scatter(b, s));
+            RET(launch_update(b, s, 0, false, defer));
+            RET(launch_scatter(b, s, kScatterJ, defer));
         }
     } else if (mode == kModeBinned) {
         for (int k = 0; k < n; ++k) {
@@ -1004,11 +1024,9 @@ static int enqueue_steps(dtb_block* b, int n, int mode)
     } else if (mode == kModeSlots || mode == kModeMasks) {
         const int g = mode == kModeSlots ? kGatherSlots : kGatherMasks;
         const int how = mode == kModeSlots ? kScatterSlots : kScatterMasks;
-        RET(launch_update(b, s, 0, false));
-        RET(launch_scatter(b, s, how));
-        for (int k = 1; k < n; ++k) {
-            RET(launch_update(b, s, g, false));
-            RET(launch_scatter(b, s, how));
+        for (int k = 0; k < n; ++k) {
+            RET(launch_update(b, s, k ? g : 0, false, defer));
+            RET(launch_scatter(b, s, how, defer));
         }
         RET(launch_gather_only(b, s, g));
     } else {
@@ -1928,10 +1946,10 @@ int dtb_block_time_kernels(dtb_block* b, int n_steps, float noise_rate, int isol
         const int g = m == kModeSlots ? kGatherSlots : kGatherMasks;
         const int how = m == kModeSlots ? kScatterSlots : (m == kModeMasks ? kScatterMasks : kScatterJ);
         for (int st = 0; st < n_steps && rc == DTB_OK && k + 6 <= n_ev; ++st) {
-            rec(k); rc = launch_update(b, b->ds, (ord && st > 0) ? g : 0, false); rec(k + 1);
+            rec(k); rc = launch_update(b, b->ds, (ord && st > 0) ? g : 0, false, can_defer(b)); rec(k + 1);
             kind.push_back(0); k += 2;
             if (rc != DTB_OK) break;
-            rec(k); rc = launch_scatter(b, b->ds, how); rec(k + 1); kind.push_back(1); k += 2;
+            rec(k); rc = launch_scatter(b, b->ds, how, can_defer(b)); rec(k + 1); kind.push_back(1); k += 2;
             done_steps++;
         }
         if (ord && rc == DTB_OK) {
@@ -2056,7 +2074,7 @@ int dtb_block_get_tuning(dtb_block* b, int key, int64_t* value)
 {
     if (!b || !value) return fail(DTB_ERR_ARG, "null argument");
     switch (key) {
-    case DTB_TUNE_SCATTER_WORDS: *value = b->scatter_wpw; break;
+    case DTB_TUNE_SCATTER_WORDS: *value = scatter_words(b); break;
     case DTB_TUNE_CHUNK: *value = b->chunk; break;
     case DTB_TUNE_PULL_THRESHOLD_PPM: *value = (int64_t)std::llround(b->pull_threshold * 1e6); break;
     case DTB_TUNE_USE_GRAPHS: *value = b->use_graphs ? 1 : 0; break;
@@ -2079,7 +2097,7 @@ int dtb_block_autotune(dtb_block* b, int n_steps, float noise_rate, float* repor
 {
     if (!b || n_steps < 2) return fail(DTB_ERR_ARG, "bad argument");
     float best_ms = 1e30f, push_ms = 0.0f, pull_ms = 0.0f, ev = 0.0f;
-    int best_w = b->scatter_wpw;
+    int best_w = scatter_words(b);
     const int pm0 = b->push_method;
     if (b->has_push) b->push_method = 1;   // atomic push first
     {   // register budget of the update kernel

@@ -71,8 +71,10 @@ struct Ctl {
     uint32_t err;                    // sticky error flags
     uint32_t pad;
     unsigned long long events;       // synaptic events propagated since creation
+    unsigned long long step_cur;     // deferred statistics: the step of the latest update, whose clock the
+                                     // scatter that follows advances
 };
-static_assert(sizeof(Ctl) == 56, "Ctl layout");
+static_assert(sizeof(Ctl) == 64, "Ctl layout");
 
 struct RunParams {
     unsigned long long run_base;
@@ -136,7 +138,7 @@ struct DevState {
     const uint16_t* qpos;       // [S] position of every push entry inside its pull row (nullable)
     // ordered push (bit-exact pull order at push cost): pending contributions per neuron
     uint32_t* slot_cnt;         // [N] contributions written since the neuron last consumed them
-    uint4* slots;               // [N][kSlotCap] {pull-row position | kind bit, 0, w.x bits, w.y bits}
+    uint4* slots;               // [kSlotCap / 2][N][2] {pull-row position | kind bit, 0, w.x bits, w.y bits}
     uint32_t* pmask;            // [N][2][kMaskWords] pull-row positions that fired (excitatory, inhibitory)
     // binned push: the scatter appends every synaptic event {neuron within bin | kind << 15, w} to the bin of
     // its postsynaptic neuron; the next update folds each bin into its chunk in shared memory
@@ -155,6 +157,8 @@ struct DevState {
     uint32_t* unmapped_nact;    // new_active of neurons whose subblock is out of range
     unsigned long long* win_spk; // [n_sub] spikes accumulated since the host last cleared them
     int stats_ext;              // 1: statistics and BOLD in k_stats (many subblocks / regions)
+    int defer;                  // 1: a scatter follows this update; its first CTAs fold the statistics,
+                                // run BOLD and advance the clock
     const int32_t* grp_ptr;     // k_stats groups: [n_groups+1] into grp_sub
     const int32_t* grp_sub;     // subblocks of every group
     const int32_t* grp_region;  // [n_groups] BOLD region of the group or -1

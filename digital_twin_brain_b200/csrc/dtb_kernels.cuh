@@ -85,6 +85,20 @@ __device__ __forceinline__ void store_J(const DevState& s, int64_t n, float4 J)
     }
 }
 
+// The same choice as an L2 policy operand: one store instruction whichever it is.
+__device__ __forceinline__ uint64_t store_policy(int keep)
+{
+    uint64_t p;
+    if (keep) asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    else asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+
+__device__ __forceinline__ void store_pair(float2* p, float x, float y, uint64_t policy)
+{
+    asm volatile("st.global.L2::cache_hint.v2.f32 [%0], {%1, %2}, %3;" :: "l"(p), "f"(x), "f"(y), "l"(policy) : "memory");
+}
+
 // Synaptic events propagated by a warp or CTA, into one of kEvParts counters.
 __device__ __forceinline__ void add_events(const DevState& s, unsigned long long ev, uint32_t key)
 {
@@ -130,9 +144,14 @@ __device__ __forceinline__ float4 gather_row(const DevState& s, const uint32_t* 
     return make_float4(a0, a1, a2, a3);
 }
 
-// Sum of one neuron's c <= kSlotCap ordered-push contributions in ascending
-// pull-row position (the order gather_row adds them).  Two terms added to +0
-// give the same float in either order, so only c >= 3 needs the ordering.
+// Where record k of neuron n's slots lies: pairs {0,1}, {2,3}, ... in planes of [N], so that the
+// first two contributions of all neurons (most of them) are 32 N contiguous bytes.
+__device__ __forceinline__ int64_t slot_at(int64_t N, int64_t n, uint32_t k)
+{
+    return ((int64_t)(k >> 1) * N + n) * 2 + (k & 1u);
+}
+
+// One ordered-push contribution {position | kind, -, w.x, w.y} added to its channels' sums.
 __device__ __forceinline__ void slot_add(uint4 v, float& a0, float& a1, float& a2, float& a3)
 {
     const float wx = __uint_as_float(v.z), wy = __uint_as_float(v.w);
@@ -140,39 +159,44 @@ __device__ __forceinline__ void slot_add(uint4 v, float& a0, float& a1, float& a
     else { a0 = __fadd_rn(a0, wx); a1 = __fadd_rn(a1, wy); }
 }
 
-// One or two contributions (already loaded): any order gives the same float.
-__device__ __forceinline__ float4 slot_pair_sum(uint4 v0, uint4 v1, uint32_t c)
+// Ascending pull-row position; the kind bit does not take part.
+__device__ __forceinline__ void slot_order(uint4& a, uint4& b)
 {
-    float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-    slot_add(v0, a0, a1, a2, a3);
-    if (c == 2u) slot_add(v1, a0, a1, a2, a3);
-    return make_float4(a0, a1, a2, a3);
+    if ((a.x & kIndexMask) > (b.x & kIndexMask)) { const uint4 t = a; a = b; b = t; }
 }
 
-__device__ __forceinline__ float4 slot_sum(const uint4* __restrict__ sl, uint32_t c)
+// Sum of one neuron's 1 <= c <= kSlotCap contributions in ascending pull-row position (the order
+// gather_row adds them); r0, r1: its first two records, loaded by the caller.  Two terms added to
+// +0 give the same float in either order; more are sorted in registers.
+__device__ __forceinline__ float4 slot_sum(const uint4* slots, int64_t N, int64_t n, uint32_t c, uint4 r0, uint4 r1)
 {
     float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-    auto add = [&](uint4 v) {
-        const float wx = __uint_as_float(v.z), wy = __uint_as_float(v.w);
-        if (v.x & kKindBit) { a2 = __fadd_rn(a2, wx); a3 = __fadd_rn(a3, wy); }
-        else { a0 = __fadd_rn(a0, wx); a1 = __fadd_rn(a1, wy); }
-    };
     if (c <= 2u) {
-        add(__ldcs(sl));
-        if (c == 2u) add(__ldcs(sl + 1));
+        slot_add(r0, a0, a1, a2, a3);
+        if (c == 2u) slot_add(r1, a0, a1, a2, a3);
+    } else if (c <= 4u) {
+        uint4 v2 = __ldcg(slots + slot_at(N, n, 2)), v3 = make_uint4(kIndexMask, 0u, 0u, 0u);
+        if (c == 4u) v3 = __ldcg(slots + slot_at(N, n, 3));
+        slot_order(r0, r1); slot_order(v2, v3); slot_order(r0, v2); slot_order(r1, v3); slot_order(r1, v2);
+        slot_add(r0, a0, a1, a2, a3); slot_add(r1, a0, a1, a2, a3); slot_add(v2, a0, a1, a2, a3);
+        if (c == 4u) slot_add(v3, a0, a1, a2, a3);
     } else {
-        uint32_t last = 0u;
-        for (uint32_t r = 0; r < c; ++r) {
-            uint4 best = make_uint4(0u, 0u, 0u, 0u);
-            uint32_t bp = 0xffffffffu;
-            for (uint32_t k = 0; k < c; ++k) {
-                const uint4 v = sl[k];
-                const uint32_t p = v.x & kIndexMask;
-                if ((r == 0u || p > last) && p < bp) { bp = p; best = v; }
-            }
-            add(best);
-            last = bp;
+        uint4 v[8] = {r0, r1};
+#pragma unroll
+        for (uint32_t k = 2; k < 8; ++k) {
+            v[k] = make_uint4(kIndexMask, 0u, 0u, 0u);
+            if (k < c) v[k] = __ldcg(slots + slot_at(N, n, k));
         }
+        // odd-even merge network for eight keys
+        slot_order(v[0], v[1]); slot_order(v[2], v[3]); slot_order(v[4], v[5]); slot_order(v[6], v[7]);
+        slot_order(v[0], v[2]); slot_order(v[1], v[3]); slot_order(v[4], v[6]); slot_order(v[5], v[7]);
+        slot_order(v[1], v[2]); slot_order(v[5], v[6]);
+        slot_order(v[0], v[4]); slot_order(v[1], v[5]); slot_order(v[2], v[6]); slot_order(v[3], v[7]);
+        slot_order(v[2], v[4]); slot_order(v[3], v[5]);
+        slot_order(v[1], v[2]); slot_order(v[3], v[4]); slot_order(v[5], v[6]);
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k)
+            if (k < c) slot_add(v[k], a0, a1, a2, a3);
     }
     return make_float4(a0, a1, a2, a3);
 }
@@ -343,12 +367,10 @@ __device__ void step_epilogue(const DevState& s, unsigned long long steps_done, 
 // group (a BOLD region with its subblocks, or a lone subblock) folds the
 // accumulators of the step just taken into the per-step rows and the window
 // totals, and runs the region's BOLD step.  Launched right after each update.
-__global__ void __launch_bounds__(256) k_stats(DevState s)
+constexpr int kStatThreads = 256;
+
+__device__ __forceinline__ void stats_group(const DevState& s, int g, unsigned long long row, bool write)
 {
-    const Ctl* ctl = s.ctl;
-    const unsigned long long row = ctl->steps_done - 1ull - ctl->run_base;   // clock already advanced
-    const bool write = row < (unsigned long long)ctl->stats_cap;
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t nact_sum = 0;
     if (g < s.n_groups) {
         double spk_sum = 0.0;
@@ -376,6 +398,31 @@ __global__ void __launch_bounds__(256) k_stats(DevState s)
     }
     const uint32_t w = __reduce_add_sync(0xffffffffu, nact_sum);
     if ((threadIdx.x & 31) == 0 && w && write) atomicAdd(s.st_nact + row, w);
+}
+
+__global__ void __launch_bounds__(kStatThreads) k_stats(DevState s)
+{
+    const unsigned long long row = s.ctl->steps_done - 1ull - s.ctl->run_base;   // clock already advanced
+    stats_group(s, blockIdx.x * blockDim.x + threadIdx.x, row, row < (unsigned long long)s.ctl->stats_cap);
+}
+
+// The same in the first CTAs of the scatter that follows a deferred update (they run beside the
+// scatter, where the update's last CTA would have run alone after a done-count); CTA 0 advances the
+// clock, which the scatter does not read (it reads step_cur).
+__device__ __forceinline__ void deferred_stats(const DevState& s)
+{
+    Ctl* ctl = s.ctl;
+    const unsigned long long step = ctl->step_cur;
+    const unsigned long long row = step - ctl->run_base;
+    const bool write = row < (unsigned long long)ctl->stats_cap;
+    stats_group(s, blockIdx.x * blockDim.x + threadIdx.x, row, write);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const uint32_t un = atomicExch(s.unmapped_nact, 0u);
+        if (un && write) atomicAdd(s.st_nact + row, un);
+        ctl->t = __fadd_rn(ctl->t, s.dt);
+        ctl->use_isyn_override = 0u;
+        ctl->steps_done = step + 1ull;
+    }
 }
 
 // ------------------------------------------------------------ samples
@@ -584,10 +631,18 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
 
     // update-phase constants (models/block.py:133-142)
     const Ctl* ctl = s.ctl;
+    if (UPDATE && s.defer && blockIdx.x == 0 && threadIdx.x == 0) {
+        const unsigned long long row = steps_done - ctl->run_base;
+        s.ctl->step_cur = steps_done;
+        if (row < (unsigned long long)ctl->stats_cap) s.st_nact[row] = 0u;
+    }
     const float t = UPDATE ? __fadd_rn(ctl->t, s.dt) : 0.0f;
     const float noise_rate = ctl->noise_rate;
     const int isolated = ctl->isolated;
     const bool use_override = UPDATE && FORCED && ctl->use_isyn_override != 0u;
+    // noise threshold: u01(x) < rate exactly when (x >> 8) < ceil(rate 2^24)
+    const uint32_t noise_thr = noise_rate >= 0.0f ? (uint32_t)fminf(ceilf(noise_rate * 16777216.0f), 16777216.0f) : 0u;
+    const uint64_t j_policy = UPDATE ? store_policy(s.j_keep) : 0ull;
     uint32_t* obits = s.bits[steps_done & 1ull];
     const uint32_t* gbits = s.bits[(steps_done - 1ull) & 1ull];
 
@@ -888,16 +943,15 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
                 sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
                 s0[j] = s1[j] = make_uint4(0u, 0u, 0u, 0u);
                 if (cnt[j]) s.slot_cnt[n] = 0u;
-                if (cnt[j] >= 1u && cnt[j] <= kSlotCap) s0[j] = __ldcs(s.slots + n * kSlotCap);
-                if (cnt[j] == 2u) s1[j] = __ldcs(s.slots + n * kSlotCap + 1);
+                if (cnt[j] >= 1u && cnt[j] <= kSlotCap) s0[j] = __ldcs(s.slots + slot_at(s.N, n, 0));
+                if (cnt[j] >= 2u && cnt[j] <= kSlotCap) s1[j] = __ldcs(s.slots + slot_at(s.N, n, 1));
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int64_t n = base + j * 32 + lane;
                 if (cnt[j] == 0u) continue;
                 if (cnt[j] > kSlotCap) ovf |= 1u << j;
-                else if (cnt[j] <= 2u) sum[j] = slot_pair_sum(s0[j], s1[j], cnt[j]);
-                else sum[j] = slot_sum(s.slots + n * kSlotCap, cnt[j]);
+                else sum[j] = slot_sum(s.slots, s.N, n, cnt[j], s0[j], s1[j]);
             }
             // overflowing rows: the warp gathers them whole, in row order
 #pragma unroll
@@ -1045,6 +1099,100 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
         }
 
         // ---- update of step `steps_done`
+        const uint32_t tcls = s.tile_cls ? __ldg(s.tile_cls + tile) : kMixedTile;   // the tile's class, or kMixedTile
+        const bool mixed = tcls == kMixedTile;
+        bool lean = false;
+        if (!FORCED && !mixed && base + kWarpNeurons <= s.N && s.j_es == 1 && (!STAGED || staged)) {
+            // A whole tile of one class, the plain form: the ALU pipe (compares, selects, bit operations)
+            // bounds the update, so no per-neuron guards, the firing masks are ballots of the predicates
+            // themselves, the minimum with V_th is the threshold test's select, and the noise test an
+            // integer compare.
+            const ParamClass p = load_class(s.pc, tcls);
+            if (p.sub >= 0 && p.sub < s.n_sub && !isnan(p.Vth)) {
+                lean = true;
+                float v_in[4], tl_in[4];
+                float4 J_in[4];
+                float* const Vp = s.V + base + lane;
+                float2* const Jp = s.J2 + base + lane;
+                float2* const Jq = Jp + s.j_ps;
+                if (!STAGED) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        v_in[j] = __ldcs(Vp + j * 32);
+                        tl_in[j] = __ldcs(s.tlast + base + lane + j * 32);
+                        if (!GATHER) {
+                            const float2 x = __ldcs(Jp + j * 32), y = __ldcs(Jq + j * 32);
+                            J_in[j] = make_float4(x.x, x.y, y.x, y.y);
+                        }
+                    }
+                }
+                uint64_t qtile = (uint64_t)tile;
+                uint32_t stream = s.stream_id;
+                if (s.member_start && p.member >= 0) {   // inside an ensemble the tile and stream are the member's own
+                    qtile = (uint64_t)((base - __ldg(s.member_start + p.member)) / kWarpNeurons);
+                    stream += (uint32_t)p.member;
+                }
+                const U4 rnd = philox4x32_10(U4{(uint32_t)(qtile * 32 + lane), stream, (uint32_t)steps_done,
+                                                (uint32_t)(steps_done >> 32)},
+                                             (uint32_t)s.seed, (uint32_t)(s.seed >> 32));
+                const uint32_t words[4] = {rnd.x, rnd.y, rnd.z, rnd.w};
+                const uint32_t thr = noise_rate >= 0.0f ? noise_thr
+                                     : p.noise > 0.0f   ? (uint32_t)fminf(ceilf(p.noise * 16777216.0f), 16777216.0f)
+                                                        : 0u;
+                if (p.sub != cur_sub) {
+                    double vw = acc_v;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) vw += __shfl_xor_sync(0xffffffffu, vw, o);
+                    if (cur_sub >= 0 && lane == 0) {
+                        atomicAdd(s.sub_spk + cur_sub, acc_spk);
+                        atomicAdd(s.sub_nact + cur_sub, acc_nact);
+                        atomicAdd(s.sub_vsum + cur_sub, vw);
+                        flushed = true;
+                    }
+                    cur_sub = p.sub; acc_spk = 0; acc_nact = 0; acc_v = 0.0;
+                }
+                uint32_t ma[4], mn[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float v, tl;
+                    float4 J;
+                    if (STAGED) {
+                        const int q = j * 32 + lane;
+                        v = reinterpret_cast<const float*>(stage_buf)[q];
+                        tl = reinterpret_cast<const float*>(stage_buf + kWarpNeurons * 4)[q];
+                        const float2 x = reinterpret_cast<const float2*>(stage_buf + kWarpNeurons * 8)[q];
+                        const float2 y = reinterpret_cast<const float2*>(stage_buf + kWarpNeurons * 16)[q];
+                        J = make_float4(x.x, x.y, y.x, y.y);
+                    } else {
+                        v = v_in[j];
+                        tl = tl_in[j];
+                        J = GATHER ? Jn[j] : J_in[j];
+                    }
+                    const float isyn = isyn_of(p, v, J);
+                    const float mainp = __fmul_rn(-p.gL, __fsub_rn(v, p.VL));
+                    const float cd = __fadd_rn(__fadd_rn(mainp, isyn), p.Iext);
+                    const float vn = __fadd_rn(v, __fmul_rn(p.rCdt, cd));
+                    const float vs = t >= __fadd_rn(tl, p.Tref) ? vn : p.Vreset;
+                    const bool a = vs >= p.Vth;
+                    const float vmin = a ? p.Vth : vs;           // torch.minimum(vs, V_th): a NaN stays NaN
+                    const bool na = (words[j] >> 8) < thr || (a && !isolated);
+                    __stcs(Vp + j * 32, vmin);
+                    store_pair(Jp + j * 32, __fmul_rn(J.x, p.decay.x), __fmul_rn(J.y, p.decay.y), j_policy);
+                    store_pair(Jq + j * 32, __fmul_rn(J.z, p.decay.z), __fmul_rn(J.w, p.decay.w), j_policy);
+                    if (a) s.tlast[base + lane + j * 32] = t;
+                    ma[j] = __ballot_sync(0xffffffffu, a);
+                    mn[j] = __ballot_sync(0xffffffffu, na);
+                    acc_v += (double)vmin;
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { acc_spk += __popc(ma[j]); acc_nact += __popc(mn[j]); }
+                if (lane == 0) {
+                    *reinterpret_cast<uint4*>(s.abits + tile * 4) = make_uint4(ma[0], ma[1], ma[2], ma[3]);
+                    *reinterpret_cast<uint4*>(obits + tile * 4) = make_uint4(mn[0], mn[1], mn[2], mn[3]);
+                }
+            }
+        }
+        if (!lean) {
         // Phase 1: every load of the lane's four neurons before any store, so their
         // latencies overlap (the stores below could alias them).  Streaming hints:
         // the state is touched once per step.
@@ -1052,8 +1200,6 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
         float v_in[4], tl_in[4];
         float4 J_in[4];
         uint32_t c_in[4];
-        const uint32_t tcls = s.tile_cls ? __ldg(s.tile_cls + tile) : kMixedTile;   // the tile's class, or kMixedTile
-        const bool mixed = tcls == kMixedTile;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int64_t n = base + j * 32 + lane;
@@ -1226,6 +1372,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
             }
             __threadfence();   // this lane's atomics before the CTA's done-count
         }
+        }
         if (STAGED) __syncwarp();   // every lane is done with the buffer before lane 0 refills it
     }
     if (flushed) __threadfence();
@@ -1270,13 +1417,13 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
         // (read before the done-count: the last CTA's epilogue clears the override flag)
         if (UPDATE && !FORCED && (s.ctl->use_isyn_override != 0u || s.gnrn != nullptr))
             atomicOr(&s.ctl->err, kErrGeneralSkipped);
-        if (UPDATE) {
+        if (UPDATE && !s.defer) {
             __threadfence();   // the CTA's statistics before its done-count
             const unsigned prev = atomicAdd(&s.ctl->done, 1u);
             sh_last = (prev == gridDim.x - 1u);
         }
     }
-    if (!UPDATE) return;
+    if (!UPDATE || s.defer) return;
     __syncthreads();
     if (sh_last) {
         __threadfence();
@@ -1286,128 +1433,117 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
 
 // ------------------------------------------------------------ push scatter
 // cuda/src/stage/presynaptic_voltage.cpp:152-266 restated for one device.
-// A warp owns `wpw` bitmask words (32*wpw presynaptic neurons).  It lists the
-// set bits in shared memory, then takes them 32 rows at a time: every lane
-// loads one row's bounds, a warp scan turns the row lengths into offsets, and
-// the lanes walk the concatenated synapses of the 32 rows together (four
-// independent index/weight loads in flight per lane), each synapse adding its
-// weight pair to the pending J with one float2 atomic.  The synapse stream is
-// read with evict-first hints so it does not push the J lines out of L2; a
-// small `wpw` keeps the rows scattered at any moment inside a narrow window
-// of neurons, whose intra-region targets then share L2-resident J lines.  No
-// CTA-wide barrier; the synaptic events (row lengths) are counted per warp.
+// A warp owns `wpw` bitmask words (32*wpw presynaptic neurons), one per lane.  Every lane with a
+// set bit loads its first row's bounds (the others' rows follow in further rounds); the warp then
+// walks the rows two at a time, four synapses of each in flight per lane, each synapse adding its
+// weight pair to the pending J with one float2 reduction.  No row lists, scans or searches: a row
+// costs its loads and four shuffles, and a small `wpw` spreads the few rows of a step over enough
+// warps that their dependent reads (word, bounds, synapses) overlap.  The synapse stream is read
+// evict-first so that it does not push J out of L2.  Rate: 180 G reductions/s while J is in L2;
+// J lines that have to come from memory make it 112 G/s (targets of a region, 384 MB of J) and
+// 31 G/s (targets anywhere).
 constexpr int kScatterThreads = 256;
 constexpr int kScatterMaxWords = 32;
-
-constexpr int kScatterUnroll = 8;   // synapses in flight per lane
+constexpr int kScatterRows = 2;                             // rows walked together
+constexpr int kScatterUnroll = 8;                           // synapses in flight per lane
 constexpr int kScatterJ = 0, kScatterSlots = 1, kScatterMasks = 2;
 
-// MINB: resident CTAs per SM the registers are budgeted for; the row lists take
-// wpw * 32 entries per warp of dynamic shared memory.
+// MINB: resident CTAs per SM the registers are budgeted for.  stat_ctas: CTAs at the front of the
+// grid that fold the statistics of a deferred update.
 template <int MODE, int MINB = 1>
-__global__ void __launch_bounds__(kScatterThreads, MINB) k_scatter(DevState s, int wpw)
+__global__ void __launch_bounds__(kScatterThreads, MINB) k_scatter(DevState s, int wpw, int stat_ctas)
 {
-    extern __shared__ uint32_t sh_rows_dyn[];
-    const unsigned long long steps_done = s.ctl->steps_done;
-    const uint32_t* __restrict__ bits = s.bits[(steps_done - 1ull) & 1ull];
+    if ((int)blockIdx.x < stat_ctas) {
+        deferred_stats(s);
+        return;
+    }
+    // the step scattered: the clock has advanced, unless this launch advances it
+    const unsigned long long step = stat_ctas ? s.ctl->step_cur : s.ctl->steps_done - 1ull;
+    const uint32_t* __restrict__ bits = (step & 1ull) ? s.bits[1] : s.bits[0];
     const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
     // rev_scatter: CTAs take the bitmask from its end, so that the first rows scattered
     // target the neurons the update wrote last, whose J lines may still be in L2
-    const int64_t bid = s.rev_scatter ? (int64_t)(gridDim.x - 1u - blockIdx.x) : (int64_t)blockIdx.x;
+    const int64_t bid = s.rev_scatter ? (int64_t)(gridDim.x - 1u - blockIdx.x) : (int64_t)blockIdx.x - stat_ctas;
     const int64_t warp_global = (bid * blockDim.x + threadIdx.x) >> 5;
     const int64_t w0 = warp_global * wpw;
-    uint32_t* rows = sh_rows_dyn + (size_t)wid * wpw * 32;
     uint32_t word = (lane < wpw && w0 + lane < s.n_words) ? __ldcs(bits + w0 + lane) : 0u;
-    // list the set bits of the window in neuron order
-    const int cnt = __popc(word);
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    int pos = incl - cnt;
-    while (word) {
-        const int b = __ffs(word) - 1;
-        word &= word - 1;
-        rows[pos++] = (uint32_t)((w0 + lane) * 32 + b);
-    }
-    __syncwarp();
-    unsigned long long warp_events = 0;
-    for (int r0 = 0; r0 < total; r0 += 32) {
-        const bool has = r0 + lane < total;
-        int64_t e0 = 0, len = 0;
-        if (has) {
-            const uint32_t pre = rows[r0 + lane];
-            e0 = __ldcs(s.qrow + pre);
-            len = __ldcs(s.qrow + pre + 1) - e0;
+    unsigned long long events = 0;
+    while (__any_sync(0xffffffffu, word != 0u)) {
+        int64_t e0 = 0;
+        int len = 0;                                                 // (a row is far below 2^31 synapses)
+        if (word) {
+            const int b = __ffs(word) - 1;
+            word &= word - 1u;
+            const int64_t* q = s.qrow + (w0 + lane) * 32 + b;
+            e0 = __ldcs(q);
+            len = (int)(__ldcs(q + 1) - e0);
+            events += (unsigned long long)len;
         }
-        // inclusive scan of the row lengths
-        int64_t off = len;
+        unsigned m = __ballot_sync(0xffffffffu, len > 0);
+        while (m) {
+            constexpr int U = kScatterUnroll / kScatterRows;
+            int64_t re[kScatterRows];
+            int rl[kScatterRows], most = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int64_t y = __shfl_up_sync(0xffffffffu, off, o);
-            if (lane >= o) off += y;
-        }
-        const int64_t T = __shfl_sync(0xffffffffu, off, 31);
-        warp_events += (unsigned long long)T;
-        const int64_t start = off - len;           // exclusive offset of this lane's row
-        for (int64_t v0 = 0; v0 < T; v0 += 32 * kScatterUnroll) {
-            uint32_t c[kScatterUnroll];
-            float2 w[kScatterUnroll];
-            uint32_t ppos[kScatterUnroll];
-            bool ok[kScatterUnroll];
-#pragma unroll
-            for (int u = 0; u < kScatterUnroll; ++u) {
-                const int64_t v = v0 + u * 32 + lane;
-                // row of v: number of rows whose inclusive offset is <= v
-                int lo = 0;
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1) {
-                    const int64_t val = __shfl_sync(0xffffffffu, off, lo + step - 1);
-                    if (val <= v) lo += step;
-                }
-                const int src = lo < 31 ? lo : 31;
-                const int64_t rs = __shfl_sync(0xffffffffu, start, src);
-                const int64_t re0 = __shfl_sync(0xffffffffu, e0, src);
-                ok[u] = v < T;
-                if (ok[u]) {
-                    const int64_t e = re0 + (v - rs);
-                    c[u] = __ldcs(s.qcol + e);
-                    if (MODE != kScatterMasks) w[u] = __ldcs(s.qw + e);
-                    if (MODE != kScatterJ) ppos[u] = __ldcs(s.qpos + e);
-                }
+            for (int r = 0; r < kScatterRows; ++r) {
+                const int l = m ? __ffs(m) - 1 : 0;
+                const bool has = m != 0u;
+                m &= m - 1u;
+                re[r] = __shfl_sync(0xffffffffu, e0, l);
+                rl[r] = __shfl_sync(0xffffffffu, len, l);
+                if (!has) rl[r] = 0;
+                most = rl[r] > most ? rl[r] : most;
             }
-            if (MODE == kScatterMasks) {
+            for (int o = lane; o < most + lane; o += 32 * U) {
+                uint32_t c[kScatterUnroll], ppos[kScatterUnroll];
+                float2 w[kScatterUnroll];
 #pragma unroll
-                for (int u = 0; u < kScatterUnroll; ++u)
-                    if (ok[u])
-                        atomicOr(s.pmask + (int64_t)(c[u] & kIndexMask) * (2 * kMaskWords) +
-                                     ((c[u] & kKindBit) ? kMaskWords : 0) + (ppos[u] >> 5),
-                                 1u << (ppos[u] & 31));
-            } else if (MODE == kScatterSlots) {
-                // every slot claim of the batch first, so their round trips overlap
-                uint32_t k[kScatterUnroll];
+                for (int r = 0; r < kScatterRows; ++r) {
+                    const uint32_t* const cp = s.qcol + re[r] + o;   // one base per row, constant offsets
+                    const float2* const wp = s.qw + re[r] + o;
+                    const uint16_t* const pp = s.qpos + re[r] + o;
 #pragma unroll
-                for (int u = 0; u < kScatterUnroll; ++u)
-                    k[u] = ok[u] ? atomicAdd(s.slot_cnt + (c[u] & kIndexMask), 1u) : kSlotCap;
+                    for (int u = 0; u < U; ++u) {
+                        c[r * U + u] = 0xffffffffu;                  // (no neuron has this index)
+                        if (o + u * 32 < rl[r]) {
+                            c[r * U + u] = __ldcs(cp + u * 32);
+                            if (MODE != kScatterMasks) w[r * U + u] = __ldcs(wp + u * 32);
+                            if (MODE != kScatterJ) ppos[r * U + u] = __ldcs(pp + u * 32);
+                        }
+                    }
+                }
+                if (MODE == kScatterMasks) {
 #pragma unroll
-                for (int u = 0; u < kScatterUnroll; ++u)
-                    if (k[u] < kSlotCap)
-                        __stcg(s.slots + (int64_t)(c[u] & kIndexMask) * kSlotCap + k[u],
-                               make_uint4(ppos[u] | (c[u] & kKindBit), 0u, __float_as_uint(w[u].x),
-                                          __float_as_uint(w[u].y)));
-            } else {
+                    for (int u = 0; u < kScatterUnroll; ++u)
+                        if (c[u] != 0xffffffffu)
+                            atomicOr(s.pmask + (int64_t)(c[u] & kIndexMask) * (2 * kMaskWords) +
+                                         ((c[u] & kKindBit) ? kMaskWords : 0) + (ppos[u] >> 5),
+                                     1u << (ppos[u] & 31));
+                } else if (MODE == kScatterSlots) {
+                    // every slot claim of the batch first, so their round trips overlap
+                    uint32_t k[kScatterUnroll];
 #pragma unroll
-                for (int u = 0; u < kScatterUnroll; ++u)
-                    if (ok[u])
-                        atomicAdd(s.J2 + (int64_t)(c[u] >> 31) * s.j_ps + (int64_t)(c[u] & kIndexMask) * s.j_es, w[u]);
+                    for (int u = 0; u < kScatterUnroll; ++u) {
+                        k[u] = kSlotCap;
+                        if (c[u] != 0xffffffffu) k[u] = atomicAdd(s.slot_cnt + (c[u] & kIndexMask), 1u);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kScatterUnroll; ++u)
+                        if (k[u] < kSlotCap)
+                            __stcg(s.slots + slot_at(s.N, c[u] & kIndexMask, k[u]),
+                                   make_uint4(ppos[u] | (c[u] & kKindBit), 0u, __float_as_uint(w[u].x), __float_as_uint(w[u].y)));
+                } else {
+#pragma unroll
+                    for (int u = 0; u < kScatterUnroll; ++u)
+                        if (c[u] != 0xffffffffu)
+                            atomicAdd(s.J2 + (int64_t)(c[u] >> 31) * s.j_ps + (int64_t)(c[u] & kIndexMask) * s.j_es, w[u]);
+                }
             }
         }
     }
-    if (lane == 0) add_events(s, warp_events, (uint32_t)warp_global);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) events += __shfl_xor_sync(0xffffffffu, events, o);
+    if (lane == 0) add_events(s, events, (uint32_t)warp_global);
 }
 
 // ------------------------------------------------------------ binned push scatter

@@ -80,12 +80,6 @@ __device__ __forceinline__ void small_barrier()
     else asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Ascending position; the kind bit does not take part.
-__device__ __forceinline__ void slot_order(uint4& a, uint4& b)
-{
-    if ((a.x & kIndexMask) > (b.x & kIndexMask)) { const uint4 t = a; a = b; b = t; }
-}
-
 // gather_row with the firing bits in shared memory.
 __device__ __forceinline__ float4 small_gather_row(const DevState& s, const uint32_t* bits, int64_t n, int lane)
 {
