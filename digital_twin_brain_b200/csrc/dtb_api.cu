@@ -182,8 +182,12 @@ struct dtb_block {
     bool bins_pending = false;    // the bins hold events not yet folded into J
     bool bins_failed = false;     // the bins could not be allocated (auto pushes with atomics)
     // graphs: one chunk graph per propagation method (push, pull rows, pull slots, ..., binned push)
-    cudaGraphExec_t graph[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    int graph_len[7] = {0, 0, 0, 0, 0, 0, 0};
+    // (and up to kMoreGraphs of other lengths per method, once a length is asked for twice in a row)
+    struct ChunkGraph { cudaGraphExec_t exec = nullptr; int n = 0, launches = 0; };
+    static constexpr int kMoreGraphs = 3;
+    ChunkGraph graph[7][1 + kMoreGraphs];
+    int last_n[7] = {0, 0, 0, 0, 0, 0, 0};
+    int next_graph[7] = {0, 0, 0, 0, 0, 0, 0};
     bool use_graphs = true;
     // small-network step loop (k_small): second-parity accumulators
     uint32_t* d_spk2 = nullptr;
@@ -210,6 +214,15 @@ struct dtb_bold {
     void* tmp_u = nullptr; void* tmp_o = nullptr;  // device staging for host pointers
     void* tmp_w = nullptr; size_t tmp_w_bytes = 0;
 };
+
+static void drop_graphs(dtb_block* b)
+{
+    for (auto& of_method : b->graph)
+        for (auto& g : of_method) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g = dtb_block::ChunkGraph();
+        }
+}
 
 template <typename T>
 static int dalloc(dtb_block* b, T** p, size_t count)
@@ -482,7 +495,7 @@ static int ensure_stats(dtb_block* b, uint32_t rows)
     b->stats_cap = cap;
     CK(cudaMemcpyAsync(&s.ctl->stats_cap, &cap, sizeof(uint32_t), cudaMemcpyHostToDevice, b->stream));
     CK(cudaStreamSynchronize(b->stream));
-    for (auto& g : b->graph) if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+    drop_graphs(b);
     return DTB_OK;
 }
 
@@ -539,7 +552,7 @@ static void destroy_block(dtb_block* b)
     if (!b) return;
     DeviceGuard g(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
-    for (auto& gr : b->graph) if (gr) cudaGraphExecDestroy(gr);
+    drop_graphs(b);
     for (void* p : b->allocs) cudaFree(p);
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
     if (b->pinned) cudaFreeHost(b->pinned);
@@ -649,13 +662,31 @@ static void step_grid(const dtb_block* b, int per_sm, unsigned& grid, int& tiles
     grid = (unsigned)((ntiles + (int64_t)tiles_per_warp * warps - 1) / ((int64_t)tiles_per_warp * warps));
 }
 
+// A kernel of the step chain (each begins with grid_follow): it may be launched while the one
+// before it on the stream still runs.
+template <typename... P, typename... A>
+static cudaError_t launch_chain(dtb_block* b, void (*k)(P...), unsigned grid, unsigned threads, size_t smem, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = b->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
 template <int G, bool U, bool F, int M>
 static void launch_step_m(dtb_block* b, const DevState& s)
 {
     unsigned grid;
     int tpw;
     step_grid(b, step_blocks_per_sm<G, U, F, M>(), grid, tpw);
-    k_step<G, U, F, M><<<grid, kStepThreads, step_dyn_smem(G), b->stream>>>(s, tpw);
+    launch_chain(b, k_step<G, U, F, M>, grid, kStepThreads, step_dyn_smem(G), s, tpw);
 }
 
 // Update with staged (bulk-copied, one tile ahead) state loads: split J planes
@@ -673,7 +704,7 @@ static void launch_step_staged(dtb_block* b, const DevState& s)
     unsigned grid;
     int tpw;
     step_grid(b, per_sm, grid, tpw);
-    k_step<0, U, F, M, true><<<grid, kStepThreads, kStagedSmem, b->stream>>>(s, tpw);
+    launch_chain(b, k_step<0, U, F, M, true>, grid, kStepThreads, kStagedSmem, s, tpw);
 }
 
 static bool staged_layout(const DevState& s) { return s.j_es == 1 && s.j_ps >= s.N && (s.j_ps % 2) == 0; }
@@ -839,18 +870,13 @@ static int launch_scatter(dtb_block* b, const DevState& s, int how = kScatterJ, 
     const int stat = defer ? std::max(1, (int)grid_for(s.n_groups, kStatThreads)) : 0;
     const unsigned grid = grid_for(warps * 32, kScatterThreads) + (unsigned)stat;
     if (grid == 0) return DTB_OK;
-    if (how == kScatterSlots) k_scatter<kScatterSlots><<<grid, kScatterThreads, 0, b->stream>>>(s, wpw, stat);
-    else if (how == kScatterMasks) k_scatter<kScatterMasks><<<grid, kScatterThreads, 0, b->stream>>>(s, wpw, stat);
-    else if (b->scatter_variant == 1) k_scatter<kScatterJ, 6><<<grid, kScatterThreads, 0, b->stream>>>(s, wpw, stat);
-    else k_scatter<kScatterJ, 4><<<grid, kScatterThreads, 0, b->stream>>>(s, wpw, stat);
+    if (how == kScatterSlots) launch_chain(b, k_scatter<kScatterSlots>, grid, kScatterThreads, 0, s, wpw, stat);
+    else if (how == kScatterMasks) launch_chain(b, k_scatter<kScatterMasks>, grid, kScatterThreads, 0, s, wpw, stat);
+    else if (b->scatter_variant == 1) launch_chain(b, k_scatter<kScatterJ, 6>, grid, kScatterThreads, 0, s, wpw, stat);
+    else launch_chain(b, k_scatter<kScatterJ, 4>, grid, kScatterThreads, 0, s, wpw, stat);
     CK(cudaGetLastError());
     b->launches++;
     return DTB_OK;
-}
-
-static void drop_graphs(dtb_block* b)
-{
-    for (auto& ge : b->graph) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
 }
 
 // ------------------------------------------------------------ binned push
@@ -1055,24 +1081,43 @@ static int enqueue_chunk_inner(dtb_block* b, int n, int mode)
 {
     // a chunk whose first update takes the I_syn override runs ungraphed (the captured graphs
     // hold the plain form of every step)
-    if (!b->use_graphs || n != b->chunk || b->stream == nullptr || b->override_live) return enqueue_steps(b, n, mode);
-    cudaGraphExec_t& ge = b->graph[mode];
-    if (!ge) {
+    if (!b->use_graphs || b->stream == nullptr || b->override_live) return enqueue_steps(b, n, mode);
+    dtb_block::ChunkGraph* slot = nullptr;
+    if (n == b->chunk) {
+        slot = &b->graph[mode][0];
+    } else {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;   // the caller may be capturing this call
+        if (cudaStreamIsCapturing(b->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone)
+            return enqueue_steps(b, n, mode);
+        for (int i = 1; i <= dtb_block::kMoreGraphs; ++i)
+            if (b->graph[mode][i].exec && b->graph[mode][i].n == n) slot = &b->graph[mode][i];
+        const bool again = b->last_n[mode] == n;   // the launches of a length asked for once cost less than its capture
+        b->last_n[mode] = n;
+        if (!slot && !again) return enqueue_steps(b, n, mode);
+        if (!slot) {
+            slot = &b->graph[mode][1 + b->next_graph[mode]];
+            b->next_graph[mode] = (b->next_graph[mode] + 1) % dtb_block::kMoreGraphs;
+            if (slot->exec) cudaGraphExecDestroy(slot->exec);
+            *slot = dtb_block::ChunkGraph();
+        }
+    }
+    if (!slot->exec) {
         cudaGraph_t g = nullptr;
         const int64_t before = b->launches;
         CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         int rc = enqueue_steps(b, n, mode);
-        b->graph_len[mode] = (int)(b->launches - before);
+        slot->launches = (int)(b->launches - before);
+        slot->n = n;
         b->launches = before;
         cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
         if (rc != DTB_OK) { if (g) cudaGraphDestroy(g); return rc; }
         if (ce != cudaSuccess) return fail(DTB_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(ce));
-        ce = cudaGraphInstantiate(&ge, g, 0);
+        ce = cudaGraphInstantiate(&slot->exec, g, 0);
         cudaGraphDestroy(g);
-        if (ce != cudaSuccess) { ge = nullptr; return fail(DTB_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ce)); }
+        if (ce != cudaSuccess) { slot->exec = nullptr; return fail(DTB_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ce)); }
     }
-    CK(cudaGraphLaunch(ge, b->stream));
-    b->launches += b->graph_len[mode];
+    CK(cudaGraphLaunch(slot->exec, b->stream));
+    b->launches += slot->launches;
     return DTB_OK;
 }
 
@@ -1817,7 +1862,7 @@ int dtb_block_set_stream(dtb_block* b, void* stream)
     if (!b) return fail(DTB_ERR_ARG, "null handle");
     DeviceGuard g(b->device);
     if (b->stream != (cudaStream_t)stream) {
-        for (auto& ge : b->graph) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
+        drop_graphs(b);
     }
     b->stream = (cudaStream_t)stream;
     return DTB_OK;
@@ -2401,7 +2446,7 @@ int dtb_block_update_property(dtb_block* b, const float* property, const float* 
     b->class_prop_base.clear();
     s.gnrn = nullptr;   // the new matrix holds every neuron's g_ui: gamma factors no longer apply
     drop_graphs(b);     // captured graphs hold the update's form for the old gnrn
-    for (auto& ge : b->graph) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
+    drop_graphs(b);
     b->override_pending = true;
     return DTB_OK;
 }
@@ -2894,7 +2939,7 @@ int dtb_block_attach_bold(dtb_block* b, int n_regions, const int32_t* sub_to_reg
     bd.E0 = E_0; bd.V0 = V_0;
     b->bold_R = n_regions;
     RET(rebuild_groups(b, sub_to_region));
-    for (auto& ge : b->graph) if (ge) { cudaGraphExecDestroy(ge); ge = nullptr; }
+    drop_graphs(b);
     return DTB_OK;
 }
 

@@ -20,6 +20,15 @@
 
 namespace dtb {
 
+// First in every kernel of the step chain: the launch may have come before the previous kernel
+// ended (programmatic dependent launch, which hides the launch itself); everything waits here for
+// the previous kernel's end, and the next one may come early in turn.
+__device__ __forceinline__ void grid_follow()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ------------------------------------------------------------ neuron math
 // Operation order of models/block.py:83-111 with round-to-nearest float32
 // intrinsics so that no multiply-add is contracted.
@@ -594,6 +603,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
                   "staged loads are for the update without gather, or with the bin fold");
     constexpr bool kBinStaged = STAGED && GATHER == kGatherBins;
     constexpr int kWarps = kStepThreads / 32;
+    grid_follow();
     extern __shared__ __align__(128) unsigned char stage_smem[];   // STAGED: [warp][2][kStageBytes]
     __shared__ __align__(8) unsigned long long stage_bar[kWarps][2];
     __shared__ int sh_sub[kWarps];
@@ -1359,15 +1369,29 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
             }
             acc_spk += cnt_spk; acc_nact += cnt_nact; acc_v += vsum_lane;
         } else {
-            // mixed subblocks in this tile: per-neuron atomics (classes re-read from L1)
+            // several subblocks in this tile: one reduction and one set of atomics per subblock and
+            // word (classes re-read from L1)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                if (!valid[j]) continue;
-                const int sb = s.pc[c_in[j]].sub;
-                if (sb >= 0 && sb < s.n_sub) {
-                    if ((act_m >> j) & 1u) atomicAdd(s.sub_spk + sb, 1u);
-                    if ((nav_m >> j) & 1u) atomicAdd(s.sub_nact + sb, 1u);
-                    atomicAdd(s.sub_vsum + sb, (double)__ldcg(s.V + base + j * 32 + lane));
+                const int sb = valid[j] ? __ldg(&s.pc[c_in[j]].sub) : -1;
+                const bool counted = sb >= 0 && sb < s.n_sub;
+                const double v = counted ? (double)__ldcg(s.V + base + j * 32 + lane) : 0.0;
+                unsigned rem = __ballot_sync(0xffffffffu, counted);
+                while (rem) {
+                    const int sr = __shfl_sync(0xffffffffu, sb, __ffs(rem) - 1);
+                    const bool mine = counted && sb == sr;
+                    const unsigned m = __ballot_sync(0xffffffffu, mine);
+                    rem &= ~m;
+                    const unsigned ma = __ballot_sync(0xffffffffu, mine && ((act_m >> j) & 1u));
+                    const unsigned mn = __ballot_sync(0xffffffffu, mine && ((nav_m >> j) & 1u));
+                    double vw = mine ? v : 0.0;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) vw += __shfl_xor_sync(0xffffffffu, vw, o);
+                    if (lane == 0) {
+                        if (ma) atomicAdd(s.sub_spk + sr, (uint32_t)__popc(ma));
+                        if (mn) atomicAdd(s.sub_nact + sr, (uint32_t)__popc(mn));
+                        atomicAdd(s.sub_vsum + sr, vw);
+                    }
                 }
             }
             __threadfence();   // this lane's atomics before the CTA's done-count
@@ -1453,6 +1477,7 @@ constexpr int kScatterJ = 0, kScatterSlots = 1, kScatterMasks = 2;
 template <int MODE, int MINB = 1>
 __global__ void __launch_bounds__(kScatterThreads, MINB) k_scatter(DevState s, int wpw, int stat_ctas)
 {
+    grid_follow();
     if ((int)blockIdx.x < stat_ctas) {
         deferred_stats(s);
         return;
