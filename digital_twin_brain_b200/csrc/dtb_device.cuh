@@ -19,7 +19,7 @@ namespace dtb {
 constexpr uint32_t kKindBit = 0x80000000u;
 constexpr uint32_t kIndexMask = 0x7fffffffu;
 constexpr int kWarpNeurons = 128;      // neurons owned by one warp in the step kernels
-constexpr uint32_t kSlotCap = 8;       // ordered-push contributions kept per neuron and step
+constexpr uint32_t kSlotCap = 12;      // ordered-push contributions kept per neuron and step (even)
 constexpr int kGatherRows = 1;         // k_step gathers whole pull rows
 constexpr int kGatherSlots = 2;        // k_step sums its ordered-push slots
 constexpr int kGatherMasks = 3;        // k_step sums the pull entries its position masks mark

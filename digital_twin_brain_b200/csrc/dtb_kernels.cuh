@@ -116,16 +116,20 @@ __device__ __forceinline__ void add_events(const DevState& s, unsigned long long
     else atomicAdd(&s.ctl->events, ev);
 }
 
-__device__ __forceinline__ bool test_bit(const uint32_t* __restrict__ bits, int64_t n)
+// (A plain load: the bitmask was written by a kernel this one may overlap the start of, so not the
+// read-only path.)
+__device__ __forceinline__ bool test_bit(const uint32_t* bits, int64_t n)
 {
-    return (__ldg(bits + (n >> 5)) >> (n & 31)) & 1u;
+    uint32_t w;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(w) : "l"(bits + (n >> 5)));
+    return (w >> (n & 31)) & 1u;
 }
 
 // ------------------------------------------------------------ pull gather
 // Sum of the weights of row n whose presynaptic neuron is set in `bits`,
 // accumulated strictly in row order from +0 (sparse.mm order). All lanes
 // return the same value.
-__device__ __forceinline__ float4 gather_row(const DevState& s, const uint32_t* __restrict__ bits, int64_t n,
+__device__ __forceinline__ float4 gather_row(const DevState& s, const uint32_t* bits, int64_t n,
                                              int lane, uint32_t& events)
 {
     const int64_t e0 = __ldg(s.prow + n);
@@ -174,39 +178,48 @@ __device__ __forceinline__ void slot_order(uint4& a, uint4& b)
     if ((a.x & kIndexMask) > (b.x & kIndexMask)) { const uint4 t = a; a = b; b = t; }
 }
 
-// Sum of one neuron's 1 <= c <= kSlotCap contributions in ascending pull-row position (the order
-// gather_row adds them); r0, r1: its first two records, loaded by the caller.  Two terms added to
-// +0 give the same float in either order; more are sorted in registers.
-__device__ __forceinline__ float4 slot_sum(const uint4* slots, int64_t N, int64_t n, uint32_t c, uint4 r0, uint4 r1)
+// More than four contributions of one neuron, sorted in registers (out of line: few lanes need it,
+// and its registers would spill the caller's).
+__device__ __noinline__ float4 slot_sum_many(const uint4* slots, int64_t N, int64_t n, uint32_t c)
 {
     float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-    if (c <= 2u) {
-        slot_add(r0, a0, a1, a2, a3);
-        if (c == 2u) slot_add(r1, a0, a1, a2, a3);
-    } else if (c <= 4u) {
-        uint4 v2 = __ldcg(slots + slot_at(N, n, 2)), v3 = make_uint4(kIndexMask, 0u, 0u, 0u);
-        if (c == 4u) v3 = __ldcg(slots + slot_at(N, n, 3));
-        slot_order(r0, r1); slot_order(v2, v3); slot_order(r0, v2); slot_order(r1, v3); slot_order(r1, v2);
-        slot_add(r0, a0, a1, a2, a3); slot_add(r1, a0, a1, a2, a3); slot_add(v2, a0, a1, a2, a3);
-        if (c == 4u) slot_add(v3, a0, a1, a2, a3);
-    } else {
-        uint4 v[8] = {r0, r1};
+    uint4 v[kSlotCap];
 #pragma unroll
-        for (uint32_t k = 2; k < 8; ++k) {
-            v[k] = make_uint4(kIndexMask, 0u, 0u, 0u);
-            if (k < c) v[k] = __ldcg(slots + slot_at(N, n, k));
-        }
-        // odd-even merge network for eight keys
-        slot_order(v[0], v[1]); slot_order(v[2], v[3]); slot_order(v[4], v[5]); slot_order(v[6], v[7]);
-        slot_order(v[0], v[2]); slot_order(v[1], v[3]); slot_order(v[4], v[6]); slot_order(v[5], v[7]);
-        slot_order(v[1], v[2]); slot_order(v[5], v[6]);
-        slot_order(v[0], v[4]); slot_order(v[1], v[5]); slot_order(v[2], v[6]); slot_order(v[3], v[7]);
-        slot_order(v[2], v[4]); slot_order(v[3], v[5]);
-        slot_order(v[1], v[2]); slot_order(v[3], v[4]); slot_order(v[5], v[6]);
-#pragma unroll
-        for (uint32_t k = 0; k < 8; ++k)
-            if (k < c) slot_add(v[k], a0, a1, a2, a3);
+    for (uint32_t k = 0; k < kSlotCap; ++k) {
+        v[k] = make_uint4(kIndexMask, 0u, 0u, 0u);
+        if (k < c) v[k] = __ldcg(slots + slot_at(N, n, k));
     }
+    // odd-even merge network for eight keys, then the rest inserted from the top
+    slot_order(v[0], v[1]); slot_order(v[2], v[3]); slot_order(v[4], v[5]); slot_order(v[6], v[7]);
+    slot_order(v[0], v[2]); slot_order(v[1], v[3]); slot_order(v[4], v[6]); slot_order(v[5], v[7]);
+    slot_order(v[1], v[2]); slot_order(v[5], v[6]);
+    slot_order(v[0], v[4]); slot_order(v[1], v[5]); slot_order(v[2], v[6]); slot_order(v[3], v[7]);
+    slot_order(v[2], v[4]); slot_order(v[3], v[5]);
+    slot_order(v[1], v[2]); slot_order(v[3], v[4]); slot_order(v[5], v[6]);
+    if (c > 8u)
+#pragma unroll
+        for (uint32_t k = 8; k < kSlotCap; ++k)
+#pragma unroll
+            for (uint32_t i = k; i > 0; --i) slot_order(v[i - 1], v[i]);
+#pragma unroll
+    for (uint32_t k = 0; k < kSlotCap; ++k)
+        if (k < c) slot_add(v[k], a0, a1, a2, a3);
+    return make_float4(a0, a1, a2, a3);
+}
+
+// Sum of one neuron's 1 <= c <= 4 contributions in ascending pull-row position (the order
+// gather_row adds them).  Two terms added to +0 give the same float in either order; v3 of c = 3
+// has the largest position.
+__device__ __forceinline__ float4 slot_sum_few(uint32_t c, uint4 v0, uint4 v1, uint4 v2, uint4 v3)
+{
+    float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
+    if (c > 2u) {
+        slot_order(v0, v1); slot_order(v2, v3); slot_order(v0, v2); slot_order(v1, v3); slot_order(v1, v2);
+    }
+    slot_add(v0, a0, a1, a2, a3);
+    if (c > 1u) slot_add(v1, a0, a1, a2, a3);
+    if (c > 2u) slot_add(v2, a0, a1, a2, a3);
+    if (c > 3u) slot_add(v3, a0, a1, a2, a3);
     return make_float4(a0, a1, a2, a3);
 }
 
@@ -826,6 +839,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
         }
         const int64_t base = tile * kWarpNeurons;
         float4 Jn[4];
+        float v_pre[4], t_pre[4];   // kGatherSlots: V and t_last, read with the slots
         if (STAGED && !kBinStaged) {
             if (!stage_off && base + kWarpNeurons <= s.N) {
                 const bool ok = stage_wait(smem_u32(&stage_bar[wid][sb]), (uint32_t)((it >> 1) & 1),
@@ -937,48 +951,59 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
                 continue;
             }
         } else if (GATHER == kGatherSlots) {
-            float4 sum[4];
-            uint32_t ovf = 0u;   // bit j: neuron j of this lane got more contributions than slots
-            // counts of the lane's four neurons, then their first two slots, all in flight together
+            // Chain of dependent reads, so everything that can be asked for together is: the tile's state
+            // and counts with the first two records of every neuron (most have at most two), then the
+            // third and fourth of the neurons that have them.
             uint32_t cnt[4];
             uint4 s0[4], s1[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int64_t n = base + j * 32 + lane;
-                cnt[j] = n < s.N ? __ldcs(s.slot_cnt + n) : 0u;
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int64_t n = base + j * 32 + lane;
-                sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                cnt[j] = 0u;
                 s0[j] = s1[j] = make_uint4(0u, 0u, 0u, 0u);
-                if (cnt[j]) s.slot_cnt[n] = 0u;
-                if (cnt[j] >= 1u && cnt[j] <= kSlotCap) s0[j] = __ldcs(s.slots + slot_at(s.N, n, 0));
-                if (cnt[j] >= 2u && cnt[j] <= kSlotCap) s1[j] = __ldcs(s.slots + slot_at(s.N, n, 1));
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int64_t n = base + j * 32 + lane;
-                if (cnt[j] == 0u) continue;
-                if (cnt[j] > kSlotCap) ovf |= 1u << j;
-                else sum[j] = slot_sum(s.slots, s.N, n, cnt[j], s0[j], s1[j]);
-            }
-            // overflowing rows: the warp gathers them whole, in row order
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                unsigned m = __ballot_sync(0xffffffffu, (ovf >> j) & 1u);
-                while (m) {
-                    const int l = __ffs(m) - 1;
-                    m &= m - 1;
-                    uint32_t ev = 0;
-                    const float4 a = gather_row(s, gbits, base + j * 32 + l, lane, ev);
-                    if (lane == l) sum[j] = a;
+                Jn[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (n < s.N) {
+                    cnt[j] = __ldcs(s.slot_cnt + n);
+                    s0[j] = __ldcs(s.slots + slot_at(s.N, n, 0));
+                    s1[j] = __ldcs(s.slots + slot_at(s.N, n, 1));
+                    Jn[j] = load_J(s, n);
+                    if (UPDATE) {
+                        v_pre[j] = __ldcs(s.V + n);
+                        t_pre[j] = __ldcs(s.tlast + n);
+                    }
                 }
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int64_t n = base + j * 32 + lane;
-                if (n < s.N) Jn[j] = add4(load_J(s, n), sum[j]);   // models/block.py:71-73
+            for (int h = 0; h < 4; h += 2) {
+                uint4 s2[2], s3[2];
+#pragma unroll
+                for (int j = h; j < h + 2; ++j) {
+                    const int64_t n = base + j * 32 + lane;
+                    s2[j - h] = s3[j - h] = make_uint4(kIndexMask, 0u, 0u, 0u);
+                    if (cnt[j]) s.slot_cnt[n] = 0u;
+                    if (cnt[j] == 3u || cnt[j] == 4u) {
+                        s2[j - h] = __ldcs(s.slots + slot_at(s.N, n, 2));
+                        if (cnt[j] == 4u) s3[j - h] = __ldcs(s.slots + slot_at(s.N, n, 3));
+                    }
+                }
+#pragma unroll
+                for (int j = h; j < h + 2; ++j) {
+                    const int64_t n = base + j * 32 + lane;
+                    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+                    const uint32_t c = cnt[j];
+                    if (c && c <= 4u) sum = slot_sum_few(c, s0[j], s1[j], s2[j - h], s3[j - h]);
+                    else if (c && c <= kSlotCap) sum = slot_sum_many(s.slots, s.N, n, c);
+                    // overflowing rows: the warp gathers them whole, in row order
+                    unsigned m = __ballot_sync(0xffffffffu, c > kSlotCap);
+                    while (m) {
+                        const int l = __ffs(m) - 1;
+                        m &= m - 1;
+                        uint32_t ev = 0;
+                        const float4 a = gather_row(s, gbits, base + j * 32 + l, lane, ev);
+                        if (lane == l) sum = a;
+                    }
+                    Jn[j] = add4(Jn[j], sum);   // models/block.py:71-73
+                }
             }
             if (!UPDATE) {
 #pragma unroll
@@ -1128,8 +1153,8 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
                 if (!STAGED) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        v_in[j] = __ldcs(Vp + j * 32);
-                        tl_in[j] = __ldcs(s.tlast + base + lane + j * 32);
+                        v_in[j] = GATHER == kGatherSlots ? v_pre[j] : __ldcs(Vp + j * 32);
+                        tl_in[j] = GATHER == kGatherSlots ? t_pre[j] : __ldcs(s.tlast + base + lane + j * 32);
                         if (!GATHER) {
                             const float2 x = __ldcs(Jp + j * 32), y = __ldcs(Jq + j * 32);
                             J_in[j] = make_float4(x.x, x.y, y.x, y.y);
@@ -1227,8 +1252,8 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
                         reinterpret_cast<float2*>(stage_buf + kWarpNeurons * 16)[k] = __ldcs(s.J2 + s.j_ps + n);
                     }
                 } else {
-                    v_in[j] = __ldcs(s.V + n);
-                    tl_in[j] = __ldcs(s.tlast + n);
+                    v_in[j] = GATHER == kGatherSlots ? v_pre[j] : __ldcs(s.V + n);
+                    tl_in[j] = GATHER == kGatherSlots ? t_pre[j] : __ldcs(s.tlast + n);
                     c_in[j] = mixed ? __ldcs(s.cls + n) : tcls;
                     if (!GATHER) J_in[j] = load_J(s, n);
                 }
@@ -1484,7 +1509,7 @@ __global__ void __launch_bounds__(kScatterThreads, MINB) k_scatter(DevState s, i
     }
     // the step scattered: the clock has advanced, unless this launch advances it
     const unsigned long long step = stat_ctas ? s.ctl->step_cur : s.ctl->steps_done - 1ull;
-    const uint32_t* __restrict__ bits = (step & 1ull) ? s.bits[1] : s.bits[0];
+    const uint32_t* bits = (step & 1ull) ? s.bits[1] : s.bits[0];
     const int lane = threadIdx.x & 31;
     // rev_scatter: CTAs take the bitmask from its end, so that the first rows scattered
     // target the neurons the update wrote last, whose J lines may still be in L2
