@@ -605,13 +605,19 @@ int net_pass(dtb_mlp* p, const float* x, const float* target, int64_t B, float* 
     g.b1 = p->w + p->o_b1; g.b2 = p->w + p->o_b2; g.b3 = p->w + p->o_b3;
     g.w3 = p->wb + p->o_W3;
     g.y = y; g.err = p->err;
-    const unsigned grid = cdiv(B, kNetRows);
+    // the most copies of a row that still fit one CTA per SM in one wave
+    const int D = cdiv(B, kNetRows / 4) <= kNetSMs ? 4 : (cdiv(B, kNetRows / 2) <= kNetSMs ? 2 : 1);
+    const unsigned grid = cdiv(B, kNetRows / D);
     if (!target) {
-        k_net<false><<<grid, kNetThreads, kNetSmem, p->stream>>>(g);
+        if (D == 4) k_net<false, 4><<<grid, kNetThreads, kNetSmem, p->stream>>>(g);
+        else if (D == 2) k_net<false, 2><<<grid, kNetThreads, kNetSmem, p->stream>>>(g);
+        else k_net<false, 1><<<grid, kNetThreads, kNetSmem, p->stream>>>(g);
     } else {
         g.Z1 = p->Z1; g.H1 = p->H1; g.H2 = p->H2; g.dZ2 = p->dZ2; g.dZ1 = p->dZ1; g.dY = p->dY;
         g.loss = p->loss;
-        k_net<true><<<grid, kNetThreads, kNetSmem, p->stream>>>(g);
+        if (D == 4) k_net<true, 4><<<grid, kNetThreads, kNetSmem, p->stream>>>(g);
+        else if (D == 2) k_net<true, 2><<<grid, kNetThreads, kNetSmem, p->stream>>>(g);
+        else k_net<true, 1><<<grid, kNetThreads, kNetSmem, p->stream>>>(g);
     }
     MCK(cudaGetLastError());
     return DTB_OK;
@@ -732,8 +738,10 @@ int dtb_mlp_create(int in_dim, int hidden, uint64_t seed, int device, dtb_mlp** 
     }
     static std::atomic<uint64_t> ready{0};   // devices whose attributes are set
     if (e == cudaSuccess && fused && !((ready.load() >> (device & 63)) & 1)) {
-        e = cudaFuncSetAttribute(k_net<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNetSmem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_net<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kNetSmem);
+        void (*const nets[])(NetArgs) = {k_net<false, 1>, k_net<false, 2>, k_net<false, 4>,
+                                         k_net<true, 1>, k_net<true, 2>, k_net<true, 4>};
+        for (auto k : nets)
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kNetSmem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k_net_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem);
         if (e == cudaSuccess) ready.fetch_or(1ull << (device & 63));
     }

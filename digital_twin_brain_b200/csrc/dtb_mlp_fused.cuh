@@ -6,11 +6,11 @@
 // 11,520 rows took 120 us for 1.6 GFLOP (two tensor-core GEMMs of 37 us, a one-column GEMM of 45).
 // Here the activations of a tile stay in TMEM and shared memory: the accumulators of both layers
 // (2 x 256 columns) fill TMEM, each hidden layer's GELU is applied as the accumulator is read, and
-// the result is written straight into the next GEMM's operand buffer, two 32-column chunks in
-// flight, so that the MMAs of one chunk run while the warps compute the next.  What bounds it is
+// the result is written straight into the next GEMM's operand buffer in 64-column chunks, the MMAs of
+// one chunk running while the warps compute the next.  What bounds it is
 // the elementwise work (erff and the three-term split, about 60 instructions per hidden unit).
-// Measured: forward of 11,520 rows 120.3 -> 18.6 us, gradient of 4,096 rows 367 -> 124 us, an Adam
-// step on 360 rows 375 -> 92 us; the error of the gradient against 64 bits 1.5e-6 -> 0.8e-6.
+// Measured: forward of 11,520 rows 120.3 -> 18.3 us, gradient of 4,096 rows 367 -> 87 us, an Adam
+// step on 360 rows 375 -> 54 us; the error of the gradient against 64 bits 1.5e-6 -> 0.8e-6.
 //
 // Weights are read as BF16 "images" in the canonical shared-memory operand order (8 x 16-byte core
 // matrices), written once when the weights change, so that a whole 256 x 256 operand arrives with
@@ -21,8 +21,9 @@
 constexpr int kNetH = 256;                 // hidden units
 constexpr int kNetMaxIn = 32;              // inputs, padded to 16 or 32
 constexpr int kNetRows = 128;              // rows per CTA (tcgen05 M)
+constexpr int kNetSMs = 148;               // SMs: one CTA each
 constexpr int kNetThreads = 256;           // warp w: TMEM lanes 32 (w % 4).., column half w / 4
-constexpr int kNetChunk = 32;              // hidden units per operand chunk
+constexpr int kNetChunk = 64;              // hidden units per operand chunk
 constexpr int kNetChunks = kNetH / kNetChunk;
 constexpr int kNetTermBytes = kNetRows * kNetChunk * 2;           // one BF16 term of a chunk
 constexpr int kNetW2Bytes = kNetH * kNetH * 2;
@@ -68,6 +69,31 @@ __device__ __forceinline__ void net_ld16(uint32_t taddr, float* v)
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// C consecutive accumulator columns of the thread's lane (C = 8, 16 or 32).
+template <int C>
+__device__ __forceinline__ void net_ld(uint32_t taddr, float* v)
+{
+    if (C == 8) {
+        uint32_t r[8];
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr) : "memory");
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+    } else {
+#pragma unroll
+        for (int c = 0; c < C; c += 16) net_ld16(taddr + (uint32_t)c, v + c);
+    }
+}
+
+template <int C>
+__device__ __forceinline__ void net_store(float* dst, const float* v)
+{
+#pragma unroll
+    for (int e = 0; e < C; e += 4) *reinterpret_cast<float4*>(dst + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+}
+
 __device__ __forceinline__ void net_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(mbar), "r"(bytes) : "memory");
@@ -76,7 +102,8 @@ __device__ __forceinline__ void net_bulk(uint32_t dst, const void* src, uint32_t
 }
 
 // Eight FP32 values as three BF16 terms (hi + mid + lo), one 16-byte store each.
-__device__ __forceinline__ void net_split8(const float* x, unsigned char* dst, int term_bytes)
+// dup > 1: also `dup_bytes` further on, and so on (the copies of a row in the other quadrants).
+__device__ __forceinline__ void net_split8(const float* x, unsigned char* dst, int term_bytes, int dup = 1, int dup_bytes = 0)
 {
     uint32_t t[3][4];
 #pragma unroll
@@ -91,7 +118,9 @@ __device__ __forceinline__ void net_split8(const float* x, unsigned char* dst, i
         }
     }
 #pragma unroll
-    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(dst + i * term_bytes) = make_uint4(t[i][0], t[i][1], t[i][2], t[i][3]);
+    for (int i = 0; i < 3; ++i)
+        for (int d = 0; d < dup; ++d)
+            *reinterpret_cast<uint4*>(dst + i * term_bytes + d * dup_bytes) = make_uint4(t[i][0], t[i][1], t[i][2], t[i][3]);
 }
 
 struct NetArgs {
@@ -110,18 +139,26 @@ struct NetArgs {
     unsigned* err;
 };
 
-constexpr int kNetOffA = kNetW2Bytes;                               // two chunk buffers x three terms
-constexpr int kNetOffX = kNetOffA + 6 * kNetTermBytes;
+constexpr int kNetOffA = kNetW2Bytes;                               // the chunk's three terms
+constexpr int kNetOffX = kNetOffA + 3 * kNetTermBytes;
 constexpr int kNetOffW1 = kNetOffX + 3 * kNetRows * kNetMaxIn * 2;
-constexpr int kNetOffF = kNetOffW1 + kNetH * kNetMaxIn * 2;         // b1, b2, w3 [256], partial y [2][128], dy [128]
+constexpr int kNetOffF = kNetOffW1 + kNetH * kNetMaxIn * 2;         // b1, b2, w3 [256], partial y [2 D][128 / D], dy
 constexpr int kNetSmem = kNetOffF + (3 * kNetH + 3 * kNetRows) * 4;
 static_assert(kNetSmem <= 227 * 1024, "shared memory of one CTA");
 
-template <bool TRAIN>
+// D: a CTA takes 128 / D rows, each of them D times in the tile (in D of the four TMEM quadrants,
+// 32 lanes each, that a warp can read): the copies cost nothing on the tensor cores, and the warps of
+// the D quadrants share a row's columns, so that a batch too small to fill the GPU with 128-row tiles
+// spends 1 / D of the time on the elementwise work that bounds it (gradient of 4,096 rows 124 -> 87 us,
+// Adam step on 360 rows 92 -> 54 us against D = 1).
+template <bool TRAIN, int D>
 __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
 {
+    constexpr int kRows = kNetRows / D;
+    constexpr int kQuads = 4 / D;                         // quadrants of distinct rows
+    constexpr int kCols = kNetChunk / (2 * D);            // columns of a chunk per thread
     extern __shared__ __align__(1024) unsigned char nsm[];
-    __shared__ __align__(8) unsigned long long bars[5];   // W1, W2, layer 1, chunk buffer 0, 1
+    __shared__ __align__(8) unsigned long long bars[4];   // W1, W2, layer 1, chunk
     __shared__ uint32_t tmem_base;
     unsigned char* sW2 = nsm;
     unsigned char* sA = nsm + kNetOffA;
@@ -133,12 +170,12 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
     float* sy = sw3 + kNetH;
     float* sdy = sy + 2 * kNetRows;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int r = (warp & 3) * 32 + lane;                 // tile row = TMEM lane
-    const int half = warp >> 2;
-    const int64_t row = (int64_t)blockIdx.x * kNetRows + r;
+    const int quad = warp & 3;
+    const int r = (quad % kQuads) * 32 + lane;            // tile row (its first copy)
+    const int grp = (quad / kQuads) * 2 + (warp >> 2);    // the thread's share of a row's columns, 0 .. 2 D - 1
+    const int64_t row = (int64_t)blockIdx.x * kRows + r;
     const bool live = row < g.B;
-    const uint32_t b_w1 = smem_addr(&bars[0]), b_w2 = smem_addr(&bars[1]), b_l1 = smem_addr(&bars[2]);
-    const uint32_t b_buf[2] = {smem_addr(&bars[3]), smem_addr(&bars[4])};
+    const uint32_t b_w1 = smem_addr(&bars[0]), b_w2 = smem_addr(&bars[1]), b_l1 = smem_addr(&bars[2]), b_ch = smem_addr(&bars[3]);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(smem_addr(&tmem_base)), "r"((uint32_t)kNetTmemCols) : "memory");
@@ -146,7 +183,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
     }
     if (tid == 0) {
 #pragma unroll
-        for (int i = 0; i < 5; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&bars[i])) : "memory");
+        for (int i = 0; i < 4; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&bars[i])) : "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         net_bulk(smem_addr(sW1), g.img1, (uint32_t)(kNetH * g.kx * 2), b_w1);
         net_bulk(smem_addr(sW2), g.img2, (uint32_t)kNetW2Bytes, b_w2);
@@ -154,23 +191,23 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
     sb1[tid] = g.b1[tid];
     sb2[tid] = g.b2[tid];
     sw3[tid] = __bfloat162float(g.w3[tid]);
-    // X: the thread's row, K groups half, half + 2, ... in three terms
+    // X: the thread's row, K groups grp, grp + 2 D, ... in three terms
     const int xterm = kNetRows * g.kx * 2;
-    for (int c = half; c < g.kx / 8; c += 2) {
+    for (int c = grp; c < g.kx / 8; c += 2 * D) {
         float v[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const int k = c * 8 + e;
             v[e] = (live && k < g.in) ? __ldg(g.x + row * g.in + k) : 0.0f;
         }
-        net_split8(v, sX + (c * (kNetRows / 8) + (r >> 3)) * 128 + (r & 7) * 16, xterm);
+        net_split8(v, sX + (c * (kNetRows / 8) + (r >> 3)) * 128 + (r & 7) * 16, xterm, D, kRows * 16);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base;
-    const uint32_t tlane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t tlane = tmem + ((uint32_t)(quad * 32) << 16);
     const uint32_t idesc = mma_idesc(kNetH);
     bool ok = true;
     if (tid == 0) {   // layer 1: Z1 = X W1^T
@@ -184,15 +221,14 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
     ok = mma_wait(b_l1, 0, kNetWait) && ok;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-    // One operand chunk: the thread's 16 values of columns 16 half.. of chunk q into buffer q & 1,
-    // then the chunk's MMAs into accumulator columns d (first: q == q0).
+    // One operand chunk: the thread's kCols values of chunk q's columns into the buffer once the MMAs
+    // that read the chunk before are done, then this chunk's MMAs into accumulator columns d (first: q == q0).
     auto chunk = [&](int q, int q0, uint32_t d, const float* v) {
-        const int buf = q & 1;
-        if (q >= 2) ok = mma_wait(b_buf[buf], (uint32_t)(((q >> 1) - 1) & 1), kNetWait) && ok;
-        unsigned char* a = sA + buf * 3 * kNetTermBytes;
+        if (q >= 1) ok = mma_wait(b_ch, (uint32_t)((q - 1) & 1), kNetWait) && ok;
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
-            net_split8(v + c * 8, a + ((half * 2 + c) * (kNetRows / 8) + (r >> 3)) * 128 + (r & 7) * 16, kNetTermBytes);
+        for (int c = 0; c < kCols / 8; ++c)
+            net_split8(v + c * 8, sA + ((grp * (kCols / 8) + c) * (kNetRows / 8) + (r >> 3)) * 128 + (r & 7) * 16, kNetTermBytes,
+                       D, kRows * 16);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
@@ -201,62 +237,53 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
             const int k8 = (q - q0) * (kNetChunk / 8);
             for (int s = 0; s < kNetChunk / 16; ++s)
                 for (int i = 0; i < 3; ++i)
-                    net_mma(d, net_desc(smem_addr(a + i * kNetTermBytes + s * 2 * (kNetRows / 8) * 128), (kNetRows / 8) * 128, 128),
+                    net_mma(d, net_desc(smem_addr(sA + i * kNetTermBytes + s * 2 * (kNetRows / 8) * 128), (kNetRows / 8) * 128, 128),
                             net_desc(smem_addr(sW2 + (k8 + 2 * s) * (kNetH / 8) * 128), (kNetH / 8) * 128, 128), idesc,
                             q > q0 || s + i > 0);
-            net_commit(b_buf[buf]);
+            net_commit(b_ch);
         }
     };
 
     // ---- layer 2: Z2 = GELU(Z1 + b1) W2^T, chunk by chunk
     if (tid == 0) ok = mma_wait(b_w2, 0, kNetWait) && ok;
     for (int q = 0; q < kNetChunks; ++q) {
-        float v[16];
-        const int c0 = q * kNetChunk + half * 16;
-        net_ld16(tlane + (uint32_t)c0, v);
+        float v[kCols];
+        const int c0 = q * kNetChunk + grp * kCols;
+        net_ld<kCols>(tlane + (uint32_t)c0, v);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] += sb1[c0 + e];
-        if (TRAIN && live) {
-            float4* z = reinterpret_cast<float4*>(g.Z1 + row * kNetH + c0);
+        for (int e = 0; e < kCols; ++e) v[e] += sb1[c0 + e];
+        if (TRAIN && live) net_store<kCols>(g.Z1 + row * kNetH + c0, v);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) z[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
-        }
-#pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = gelu(v[e]);
-        if (TRAIN && live) {
-            float4* z = reinterpret_cast<float4*>(g.H1 + row * kNetH + c0);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) z[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
-        }
+        for (int e = 0; e < kCols; ++e) v[e] = gelu(v[e]);
+        if (TRAIN && live) net_store<kCols>(g.H1 + row * kNetH + c0, v);
         chunk(q, 0, tmem + kNetH, v);
     }
-    ok = mma_wait(b_buf[1], (uint32_t)(((kNetChunks - 1) >> 1) & 1), kNetWait) && ok;
+    ok = mma_wait(b_ch, (uint32_t)((kNetChunks - 1) & 1), kNetWait) && ok;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (TRAIN && tid == 0) net_bulk(smem_addr(sW2), g.img2t, (uint32_t)kNetW2Bytes, b_w2);   // every MMA that read W2 is done
 
     // ---- output: y = GELU(Z2 + b2) . w3 + b3
     float p = 0.0f;
-    for (int c = 0; c < kNetH / 2; c += 16) {
-        float v[16];
-        const int c0 = half * (kNetH / 2) + c;
-        net_ld16(tlane + (uint32_t)(kNetH + c0), v);
+    for (int q = 0; q < kNetChunks; ++q) {
+        float v[kCols];
+        const int c0 = q * kNetChunk + grp * kCols;
+        net_ld<kCols>(tlane + (uint32_t)(kNetH + c0), v);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
+        for (int e = 0; e < kCols; ++e) {
             v[e] = gelu(v[e] + sb2[c0 + e]);
             p = fmaf(v[e], sw3[c0 + e], p);
         }
-        if (TRAIN && live) {
-            float4* z = reinterpret_cast<float4*>(g.H2 + row * kNetH + c0);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) z[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
-        }
+        if (TRAIN && live) net_store<kCols>(g.H2 + row * kNetH + c0, v);
     }
-    sy[half * kNetRows + r] = p;
+    sy[grp * kRows + r] = p;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (tid < kNetRows) {   // threads 0..127: tile row tid
-        const float y = sy[tid] + sy[kNetRows + tid] + g.b3[0];
+    if (tid < kRows) {   // threads 0 .. kRows - 1: tile row tid (grp 0 of the first quadrants)
+        float y = sy[tid];
+#pragma unroll
+        for (int i = 1; i < 2 * D; ++i) y += sy[i * kRows + tid];
+        y += g.b3[0];
         if (live && g.y) g.y[row] = y;
         if (TRAIN) {        // loss = mean((y - t)^2), dy = 2 (y - t) / B
             const float d = live ? y - g.target[row] : 0.0f;
@@ -275,33 +302,29 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
         // ---- dZ2 = dy w3 GELU'(Z2), and dH1 = dZ2 W2 over Z1's accumulator columns
         if (tid == 0) ok = mma_wait(b_w2, 1, kNetWait) && ok;
         for (int q = kNetChunks; q < 2 * kNetChunks; ++q) {
-            float v[16];
-            const int c0 = (q - kNetChunks) * kNetChunk + half * 16;
-            net_ld16(tlane + (uint32_t)(kNetH + c0), v);
+            float v[kCols];
+            const int c0 = (q - kNetChunks) * kNetChunk + grp * kCols;
+            net_ld<kCols>(tlane + (uint32_t)(kNetH + c0), v);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) v[e] = (dy * sw3[c0 + e]) * gelu_grad(v[e] + sb2[c0 + e]);
-            if (live) {
-                float4* z = reinterpret_cast<float4*>(g.dZ2 + row * kNetH + c0);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) z[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
-            }
+            for (int e = 0; e < kCols; ++e) v[e] = (dy * sw3[c0 + e]) * gelu_grad(v[e] + sb2[c0 + e]);
+            if (live) net_store<kCols>(g.dZ2 + row * kNetH + c0, v);
             chunk(q, kNetChunks, tmem, v);
         }
-        ok = mma_wait(b_buf[1], (uint32_t)(((2 * kNetChunks - 1) >> 1) & 1), kNetWait) && ok;
+        ok = mma_wait(b_ch, (uint32_t)((2 * kNetChunks - 1) & 1), kNetWait) && ok;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int q = 0; q < kNetChunks; ++q) {   // dZ1 = dH1 GELU'(Z1), Z1 as this thread wrote it above
-            float v[16];
-            const int c0 = q * kNetChunk + half * 16;
-            net_ld16(tlane + (uint32_t)c0, v);
+            float v[kCols];
+            const int c0 = q * kNetChunk + grp * kCols;
+            net_ld<kCols>(tlane + (uint32_t)c0, v);
             if (live) {
                 const float4* z1 = reinterpret_cast<const float4*>(g.Z1 + row * kNetH + c0);
-                float4* z = reinterpret_cast<float4*>(g.dZ1 + row * kNetH + c0);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float4 a = z1[e];
-                    z[e] = make_float4(v[4 * e] * gelu_grad(a.x), v[4 * e + 1] * gelu_grad(a.y),
-                                       v[4 * e + 2] * gelu_grad(a.z), v[4 * e + 3] * gelu_grad(a.w));
+                for (int e = 0; e < kCols; e += 4) {
+                    const float4 a = z1[e / 4];
+                    v[e] *= gelu_grad(a.x); v[e + 1] *= gelu_grad(a.y);
+                    v[e + 2] *= gelu_grad(a.z); v[e + 3] *= gelu_grad(a.w);
                 }
+                net_store<kCols>(g.dZ1 + row * kNetH + c0, v);
             }
         }
     }
@@ -309,7 +332,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
         if (g.err) atomicOr(g.err, 1u);
         mma_wait(b_w1, 0, 1u << 24);
         mma_wait(b_w2, TRAIN ? 1u : 0u, 1u << 24);
-        mma_wait(b_buf[1], (uint32_t)((((TRAIN ? 2 : 1) * kNetChunks - 1) >> 1) & 1), 1u << 24);
+        mma_wait(b_ch, (uint32_t)(((TRAIN ? 2 : 1) * kNetChunks - 1) & 1), 1u << 24);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
