@@ -167,8 +167,8 @@ struct dtb_block {
     double pull_threshold = 0.05;
     int chunk = 32;
     int scatter_wpw = 0;          // bitmask words per warp in the push scatter (0: by network size)
-    int scatter_variant = 0;      // 0: registers unbounded, 1: budgeted for 6 resident CTAs per SM
-    int step_variant = 3;         // 0: 2 resident CTAs/SM register budget, 1: 3; 2..4: staged, 2..4 CTAs/SM
+    int scatter_variant = -1;     // 1: targets prefetched into L2 before their reductions, 0: not, -1: by network size
+    int step_variant = 2;         // 0: 2 resident CTAs/SM register budget, 1: 3; 2..4: staged, 2..4 CTAs/SM
     // ordered push (bit-exact pull through per-neuron slots)
     bool has_qpos = false;
     int pull_method = 0;          // 0: auto, 1: row gather, 2: ordered push (slots), 3: (masks), 4: streamed gather
@@ -376,8 +376,6 @@ static int alloc_state(dtb_block* b)
     RET(dalloc(b, &s.ctl, 1));
     RET(dalloc(b, &s.ev_part, kEvParts));
     RET(dalloc(b, &s.unmapped_nact, 1));
-    RET(dalloc(b, &b->d_unmapped2, 1));
-    CK(cudaMemsetAsync(b->d_unmapped2, 0, sizeof(uint32_t), b->stream));
     RET(dalloc(b, &b->d_err, 4));
     CK(cudaMemsetAsync(s.J2, 0, sizeof(float2) * 2 * (size_t)jps, b->stream));
     CK(cudaMemsetAsync(s.tlast, 0, sizeof(float) * (size_t)N, b->stream));
@@ -414,12 +412,11 @@ static int upload_class_tables(dtb_block* b)
         RET(dalloc(b, &s.sub_nact, (size_t)cap));
         RET(dalloc(b, &s.sub_vsum, (size_t)cap));
         RET(dalloc(b, &s.win_spk, (size_t)cap));
-        RET(dalloc(b, &b->d_spk2, (size_t)cap));
-        RET(dalloc(b, &b->d_nact2, (size_t)cap));
-        RET(dalloc(b, &b->d_vsum2, (size_t)cap));
-        CK(cudaMemsetAsync(b->d_spk2, 0, sizeof(uint32_t) * cap, b->stream));
-        CK(cudaMemsetAsync(b->d_nact2, 0, sizeof(uint32_t) * cap, b->stream));
-        CK(cudaMemsetAsync(b->d_vsum2, 0, sizeof(double) * cap, b->stream));
+        RET(dalloc(b, &b->d_vsum2, (size_t)2 * cap + 1));   // and the counts behind the sums
+        CK(cudaMemsetAsync(b->d_vsum2, 0, sizeof(double) * ((size_t)2 * cap + 1), b->stream));
+        b->d_spk2 = reinterpret_cast<uint32_t*>(b->d_vsum2 + cap);
+        b->d_nact2 = b->d_spk2 + cap;
+        b->d_unmapped2 = b->d_nact2 + cap;
         CK(cudaMemsetAsync(s.win_spk, 0, sizeof(unsigned long long) * cap, b->stream));
         CK(cudaMemsetAsync(s.sub_spk, 0, sizeof(uint32_t) * cap, b->stream));
         CK(cudaMemsetAsync(s.sub_nact, 0, sizeof(uint32_t) * cap, b->stream));
@@ -601,15 +598,14 @@ static int rebuild_groups(dtb_block* b, const int32_t* sub_to_region)
         for (int i = 0; i < n_sub; ++i) { sub.push_back(i); reg.push_back(-1); }
     }
     CK(cudaStreamSynchronize(b->stream));   // the previous tables are no longer in use
-    dfree(b, s.grp_ptr); dfree(b, s.grp_sub); dfree(b, s.grp_region);
-    int32_t *dp = nullptr, *ds = nullptr, *dr = nullptr;
-    RET(dalloc(b, &dp, ptr.size()));
-    RET(dalloc(b, &ds, std::max<size_t>(1, sub.size())));
-    RET(dalloc(b, &dr, std::max<size_t>(1, reg.size())));
-    CK(cudaMemcpy(dp, ptr.data(), sizeof(int32_t) * ptr.size(), cudaMemcpyHostToDevice));
-    if (!sub.empty()) CK(cudaMemcpy(ds, sub.data(), sizeof(int32_t) * sub.size(), cudaMemcpyHostToDevice));
-    if (!reg.empty()) CK(cudaMemcpy(dr, reg.data(), sizeof(int32_t) * reg.size(), cudaMemcpyHostToDevice));
-    s.grp_ptr = dp; s.grp_sub = ds; s.grp_region = dr;
+    dfree(b, s.grp_ptr);
+    std::vector<int32_t> all(ptr);           // one table: pointers, subblocks, regions
+    all.insert(all.end(), sub.begin(), sub.end());
+    all.insert(all.end(), reg.begin(), reg.end());
+    int32_t* dp = nullptr;
+    RET(dalloc(b, &dp, all.size() + 1));
+    if (!all.empty()) CK(cudaMemcpy(dp, all.data(), sizeof(int32_t) * all.size(), cudaMemcpyHostToDevice));
+    s.grp_ptr = dp; s.grp_sub = dp + ptr.size(); s.grp_region = s.grp_sub + sub.size();
     s.n_groups = (int)reg.size();
     b->grp_n_sub = n_sub;
     return DTB_OK;
@@ -862,6 +858,14 @@ static int scatter_words(const dtb_block* b)
     return w;
 }
 
+// Prefetched targets pay once J no longer fits L2 (1.2e7 neurons, 195 MB of J: scatter 195 -> 180 us,
+// step 279 -> 267); while it does they only cost (1e6: 17.0 -> 21.3 us).
+static int scatter_form(const dtb_block* b)
+{
+    if (b->scatter_variant >= 0) return b->scatter_variant;
+    return 16 * b->N > ((int64_t)126 << 20) ? 1 : 0;
+}
+
 // how: kScatterJ (push), kScatterSlots / kScatterMasks (ordered push)
 static int launch_scatter(dtb_block* b, const DevState& s, int how = kScatterJ, bool defer = false)
 {
@@ -872,7 +876,7 @@ static int launch_scatter(dtb_block* b, const DevState& s, int how = kScatterJ, 
     if (grid == 0) return DTB_OK;
     if (how == kScatterSlots) launch_chain(b, k_scatter<kScatterSlots>, grid, kScatterThreads, 0, s, wpw, stat);
     else if (how == kScatterMasks) launch_chain(b, k_scatter<kScatterMasks>, grid, kScatterThreads, 0, s, wpw, stat);
-    else if (b->scatter_variant == 1) launch_chain(b, k_scatter<kScatterJ, 6>, grid, kScatterThreads, 0, s, wpw, stat);
+    else if (scatter_form(b) == 1) launch_chain(b, k_scatter<kScatterJ, 4, true>, grid, kScatterThreads, 0, s, wpw, stat);
     else launch_chain(b, k_scatter<kScatterJ, 4>, grid, kScatterThreads, 0, s, wpw, stat);
     CK(cudaGetLastError());
     b->launches++;
@@ -2126,7 +2130,7 @@ int dtb_block_get_tuning(dtb_block* b, int key, int64_t* value)
     case DTB_TUNE_STEP_VARIANT: *value = b->step_variant; break;
     case DTB_TUNE_PULL_METHOD: *value = b->pull_method; break;
     case DTB_TUNE_J_CACHE: *value = b->ds.j_keep; break;
-    case DTB_TUNE_SCATTER_VARIANT: *value = b->scatter_variant; break;
+    case DTB_TUNE_SCATTER_VARIANT: *value = scatter_form(b); break;
     case DTB_TUNE_PUSH_METHOD: *value = b->push_method; break;
     case DTB_TUNE_STAGE_WAIT_LIMIT: *value = b->ds.stage_wait_limit; break;
     case DTB_TUNE_SCATTER_REVERSE: *value = b->ds.rev_scatter; break;
@@ -2160,7 +2164,7 @@ int dtb_block_autotune(dtb_block* b, int n_steps, float noise_rate, float* repor
     }
     if (b->has_push) {
         const int cand[6] = {1, 2, 4, 8, 16, 32};
-        int best_sv = b->scatter_variant;
+        int best_sv = scatter_form(b);
         for (int sv = 0; sv < 2; ++sv)
             for (int w : cand) {
                 b->scatter_wpw = w;

@@ -1497,9 +1497,10 @@ constexpr int kScatterRows = 2;                             // rows walked toget
 constexpr int kScatterUnroll = 8;                           // synapses in flight per lane
 constexpr int kScatterJ = 0, kScatterSlots = 1, kScatterMasks = 2;
 
-// MINB: resident CTAs per SM the registers are budgeted for.  stat_ctas: CTAs at the front of the
+// MINB: resident CTAs per SM the registers are budgeted for.  PREFETCH: the batch's J sectors are
+// fetched into L2 first, where the reductions then find them.  stat_ctas: CTAs at the front of the
 // grid that fold the statistics of a deferred update.
-template <int MODE, int MINB = 1>
+template <int MODE, int MINB = 1, bool PREFETCH = false>
 __global__ void __launch_bounds__(kScatterThreads, MINB) k_scatter(DevState s, int wpw, int stat_ctas)
 {
     grid_follow();
@@ -1583,6 +1584,13 @@ __global__ void __launch_bounds__(kScatterThreads, MINB) k_scatter(DevState s, i
                             __stcg(s.slots + slot_at(s.N, c[u] & kIndexMask, k[u]),
                                    make_uint4(ppos[u] | (c[u] & kKindBit), 0u, __float_as_uint(w[u].x), __float_as_uint(w[u].y)));
                 } else {
+                    if (PREFETCH) {
+#pragma unroll
+                        for (int u = 0; u < kScatterUnroll; ++u)
+                            if (c[u] != 0xffffffffu)
+                                asm volatile("prefetch.global.L2 [%0];"
+                                             :: "l"(s.J2 + (int64_t)(c[u] >> 31) * s.j_ps + (int64_t)(c[u] & kIndexMask) * s.j_es));
+                    }
 #pragma unroll
                     for (int u = 0; u < kScatterUnroll; ++u)
                         if (c[u] != 0xffffffffu)

@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_grad(GradArgs g)
     for (int64_t r0 = r_begin; r0 < r_end; r0 += kGradStage, ++st) {
         if (st > 0) ok = mma_wait(mb, (uint32_t)((st - 1) & 1), kNetWait) && ok;   // the operands are free again
         // H1^T: thread = column i, eight row groups
-#pragma unroll 2
+#pragma unroll 4
         for (int c = 0; c < kGradStage / 8; ++c) {
             float v[8];
 #pragma unroll
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_grad(GradArgs g)
             net_split8(v, gsm + kGradOffB + (c * (kNetH / 8) + (tid >> 3)) * 128 + (tid & 7) * 16, kGradB);
         }
         // dZ2^T, dZ1^T: thread = output column, half of the row groups; column sums
-#pragma unroll 2
+#pragma unroll 4
         for (int cc = 0; cc < kGradStage / 16; ++cc) {
             const int c = og * (kGradStage / 16) + cc;
             float v[8], u[8];

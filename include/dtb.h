@@ -207,7 +207,10 @@ int dtb_block_step_forced(dtb_block* b, float noise_rate, int isolated, int mode
 int dtb_block_time_kernels(dtb_block* b, int n_steps, float noise_rate, int isolated, int mode, float* out_ms);
 
 /* Schedule knobs (new: the reference has a fixed launch shape per kernel).
- * DTB_TUNE_SCATTER_WORDS   bitmask words per warp in the push scatter (1..32)
+ * DTB_TUNE_SCATTER_WORDS   bitmask words per warp in the push scatter (1..32; until
+ *                          set, 1, 2 or 4 by the network's size)
+ * Networks of up to 12,288 neurons run their steps in one cluster launch unless one of
+ * the schedule keys below was set (the results are the same).
  * DTB_TUNE_CHUNK           steps per captured CUDA graph (1..4096)
  * DTB_TUNE_PULL_THRESHOLD_PPM  activity fraction (parts per million of the
  *                          neurons propagating per step) above which
@@ -217,7 +220,7 @@ int dtb_block_time_kernels(dtb_block* b, int n_steps, float noise_rate, int isol
  *                          CTAs per SM (no spills), 1 = three, 2, 3 and 4 =
  *                          two, three and four with the state of the next
  *                          tile bulk-copied to shared memory while the
- *                          current one computes (default 3; the results are
+ *                          current one computes (default 2; the results are
  *                          bit-identical every way; a network whose J planes
  *                          do not allow the copies runs variant 0 or 1)
  * DTB_TUNE_PULL_METHOD     how DTB_MODE_PULL propagates (bit-identical every
@@ -234,8 +237,9 @@ int dtb_block_time_kernels(dtb_block* b, int n_steps, float noise_rate, int isol
  *                          neurons propagate, else the streamed gather
  * DTB_TUNE_J_CACHE         0 = the update streams J (evict first), 1 = its J
  *                          stores keep normal L2 priority for the scatter
- * DTB_TUNE_SCATTER_VARIANT push scatter registers: 0 = unbounded, 1 = budgeted
- *                          for six resident CTAs per SM
+ * DTB_TUNE_SCATTER_VARIANT push scatter: 1 = the targets of a batch are prefetched into
+ *                          L2 before their reductions, 0 = not (until set, 1 for networks
+ *                          whose J exceeds L2)
  * DTB_TUNE_PUSH_METHOD     how DTB_MODE_PUSH adds the weights of firing rows
  *                          (the order of the float additions differs, the sums
  *                          agree to rounding): 1 = one float2 atomic into J per
