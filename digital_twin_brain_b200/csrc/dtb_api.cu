@@ -2939,8 +2939,8 @@ int dtb_block_attach_bold(dtb_block* b, int n_regions, const int32_t* sub_to_reg
     bd.region_n = drn;
     bd.s = st; bd.q = st + n_regions; bd.v = st + 2 * n_regions; bd.f = st + 3 * n_regions;
     bd.act = st + 4 * n_regions; bd.out = st + 5 * n_regions;
-    bd.c = bold_const(epsilon, tao_s, tao_f, tao_0, alpha, E_0, delta_t);
-    bd.E0 = E_0; bd.V0 = V_0;
+    bd.epsilon = epsilon; bd.tao_s = tao_s; bd.tao_f = tao_f; bd.tao_0 = tao_0; bd.div_alpha = 1.0 / alpha;
+    bd.E0 = E_0; bd.V0 = V_0; bd.delta_t = delta_t;
     b->bold_R = n_regions;
     RET(rebuild_groups(b, sub_to_region));
     drop_graphs(b);

@@ -93,12 +93,11 @@ struct BoldConst {
 };
 
 struct BoldDev {
-    BoldConst c;
     int n_regions;               // 0: no BOLD attached
     const int32_t* sub_region;   // [n_sub] -> region or -1
     const double* region_n;      // [R] neurons in region
     double* s; double* q; double* v; double* f; double* act; double* out;   // [R]
-    double E0, V0;
+    double epsilon, tao_s, tao_f, tao_0, div_alpha, E0, V0, delta_t;
 };
 
 struct DevState {

@@ -11,9 +11,9 @@
 //               the pending J.  The pull gather of step k is fused with the
 //               update of step k+1 (k_step<true,true>), so a run of n pull
 //               steps is update, n-1 fused kernels and one gather-only kernel.
-// The last CTA of every update kernel folds the per-subblock statistics,
-// runs the per-region BOLD step when one is attached, and advances the
-// device clock (steps_done, t) — no extra launch per step.
+// The per-subblock statistics, the per-region BOLD step when one is attached and the device clock
+// (steps_done, t) take no launch of their own: the first CTAs of the scatter that follows an update
+// fold them, and where none follows the update's last CTA does (many subblocks: k_stats).
 #pragma once
 
 #include "dtb_device.cuh"
@@ -291,7 +291,7 @@ __device__ __forceinline__ void bold_powers(const BoldConst& c, double v, double
 }
 
 // models/bold_model_pytorch.py:43-78 in float64 (q before v before f_in before s, f_in clamped
-// at 0).  Three pow calls and six divisions made a step fp64-issue bound; with the products, one
+// at 0) for windows of steps.  Three pow calls and six divisions made a step fp64-issue bound; with the products, one
 // exp and the reciprocals it has one division.
 __device__ __forceinline__ void bold_qv(const BoldConst& c, double f, double ext, double& q, double& v)
 {
@@ -312,12 +312,20 @@ __device__ __forceinline__ void bold_fs(const BoldConst& c, double eu, double& f
     s = fma(ds, c.dt, s);
 }
 
-// One step of region r with input u.
+// One step of region r with input u, for networks with BOLD attached: the reference's own operations
+// (pow, divisions), so that a bit-exact run's signal keeps its last bit; it runs beside the scatter.
 __device__ __forceinline__ void bold_region_step(const BoldDev& b, int r, double u)
 {
     double fi = b.f[r], si = b.s[r], qi = b.q[r], vi = b.v[r];
-    bold_qv(b.c, fi, fi > 0.0 ? bold_extraction(b.c, fi) : 0.0, qi, vi);
-    bold_fs(b.c, u * b.c.eps, fi, si);
+    const double ds = ((b.epsilon * u) - si / b.tao_s) - (fi - 1.0) / b.tao_f;
+    const double qpart = fi > 0.0 ? (1.0 - pow(1.0 - b.E0, 1.0 / fi)) : 1.0;
+    const double dq = (((fi * qpart) / b.E0) - qi * pow(vi, b.div_alpha - 1.0)) / b.tao_0;
+    qi = qi + dq * b.delta_t;
+    const double dv = (fi - pow(vi, b.div_alpha)) / b.tao_0;
+    vi = vi + dv * b.delta_t;
+    fi = fi + si * b.delta_t;
+    fi = fi > 0.0 ? fi : 0.0;
+    si = si + ds * b.delta_t;
     b.s[r] = si; b.q[r] = qi; b.v[r] = vi; b.f[r] = fi;
     b.out[r] = b.V0 * ((7.0 * b.E0 * (1.0 - qi) + 2.0 * (1.0 - qi / vi)) + (2.0 * b.E0 - 0.2) * (1.0 - vi));
 }

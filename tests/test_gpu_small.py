@@ -19,7 +19,7 @@ def _same(a, b):
 
 
 @pytest.mark.parametrize("rate", [0.01, 0.09])
-@pytest.mark.parametrize("N,K", [(2, 1), (31, 8), (33, 20), (384, 60), (385, 60), (1000, 130), (3072, 40), (3073, 40),
+@pytest.mark.parametrize("N,K", [(2, 1), (31, 8), (33, 20), (384, 60), (385, 60), (1000, 130), (1900, 20), (2600, 20), (3072, 40), (3073, 40),
                                  (12288, 25), (12289, 25)])
 def test_small_loop_equals_row_gather(N, K, rate):
     spec = synthetic.single_block(N, K, gen_seed=N, g_ui=(0.02, 0.001, 0.1, 0.005))
