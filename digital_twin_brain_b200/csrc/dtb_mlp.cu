@@ -507,6 +507,7 @@ struct dtb_mlp {
     float* v = nullptr;
     float* loss = nullptr;         // device scalar: g[n_params]
     int64_t cap = 0;               // batch capacity of the activation buffers
+    float* act = nullptr;          // the allocation that holds them (fused kernels)
     float *Z1 = nullptr, *H1 = nullptr, *Z2 = nullptr, *H2 = nullptr, *Y = nullptr;
     float *dY = nullptr, *dH2 = nullptr, *dZ2 = nullptr, *dH1 = nullptr, *dZ1 = nullptr;
     int64_t t = 0;                 // Adam step
@@ -581,6 +582,17 @@ int check_err(dtb_mlp* p)
 int ensure_cap(dtb_mlp* p, int64_t B)
 {
     if (B <= p->cap) return DTB_OK;
+    if (p->img) {   // the fused kernels' buffers, in one allocation
+        if (p->act) cudaFree(p->act);
+        p->act = nullptr;
+        p->cap = 0;
+        const size_t n = (size_t)B * p->H;
+        MCK(cudaMalloc(&p->act, sizeof(float) * (5 * n + (size_t)B)));
+        p->Z1 = p->act; p->H1 = p->Z1 + n; p->H2 = p->H1 + n; p->dZ2 = p->H2 + n; p->dZ1 = p->dZ2 + n;
+        p->dY = p->dZ1 + n;
+        p->cap = B;
+        return DTB_OK;
+    }
     float** bufs[] = {&p->Z1, &p->H1, &p->Z2, &p->H2, &p->dH2, &p->dZ2, &p->dH1, &p->dZ1};
     for (float** b : bufs) { if (*b) cudaFree(*b); *b = nullptr; }
     if (p->Y) cudaFree(p->Y);
@@ -769,6 +781,7 @@ int dtb_mlp_destroy(dtb_mlp* p)
     int prev = -1;
     cudaGetDevice(&prev);
     cudaSetDevice(p->device);
+    if (p->act) { cudaFree(p->act); p->Z1 = p->H1 = p->H2 = p->dZ2 = p->dZ1 = p->dY = nullptr; }
     void* bufs[] = {p->mem, p->mem2, p->Z1, p->H1, p->Z2, p->H2, p->Y,
                     p->dY, p->dH2, p->dZ2, p->dH1, p->dZ1};
     for (void* b : bufs) if (b) cudaFree(b);
