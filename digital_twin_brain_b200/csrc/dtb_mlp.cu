@@ -497,7 +497,7 @@ struct dtb_mlp {
     int in = 0, H = 0;
     int64_t n_params = 0;
     int64_t o_W1, o_b1, o_W2, o_b2, o_W3, o_b3;
-    void *mem = nullptr, *mem2 = nullptr;   // the allocations that hold everything up to the activations
+    void* tail = nullptr;          // the allocation of the operand images and the error flag
     float* w = nullptr;            // FP32 master [n_params]
     __nv_bfloat16* wb = nullptr;   // BF16 compute copy
     __nv_bfloat16* img = nullptr;  // fused kernels: W2, W2^T and W1 as operand images (null: layer by layer)
@@ -728,29 +728,28 @@ int dtb_mlp_create(int in_dim, int hidden, uint64_t seed, int device, dtb_mlp** 
     for (int64_t i = 0; i < (int64_t)hidden * in_dim; ++i) w[(size_t)(p->o_W1 + i)] = (2.0f * uni() - 1.0f) * a1;
     for (int64_t i = 0; i < (int64_t)hidden * hidden; ++i) w[(size_t)(p->o_W2 + i)] = (2.0f * uni() - 1.0f) * a2;
     for (int64_t i = 0; i < hidden; ++i) w[(size_t)(p->o_W3 + i)] = (2.0f * uni() - 1.0f) * a2;
-    // two allocations (each under 1 MB, which the driver serves from a shared block): masters, gradients
-    // and loss, first moments; second moments, BF16 copy, operand images, error flag
     const bool fused = hidden == kNetH && in_dim <= kNetMaxIn;
-    const size_t f4 = (sizeof(float) * (size_t)(o + 1) + 255) & ~(size_t)255;
-    const size_t f2 = (sizeof(__nv_bfloat16) * (size_t)o + 255) & ~(size_t)255;
+    const size_t f4 = sizeof(float) * (size_t)o;
     const size_t fi = fused ? sizeof(__nv_bfloat16) * (size_t)(2 * kNetImgW2 + kNetH * kNetMaxIn) : 0;
-    char *mem = nullptr, *mem2 = nullptr;
-    cudaError_t e = cudaMalloc(&mem, 3 * f4);
-    p->mem = mem;
-    if (e == cudaSuccess) e = cudaMalloc(&mem2, f4 + f2 + fi + 256);
-    p->mem2 = mem2;
+    unsigned char* tail = nullptr;   // operand images, then the error flag
+    cudaError_t e = cudaMalloc(&p->w, f4);
+    if (e == cudaSuccess) e = cudaMalloc(&p->wb, sizeof(__nv_bfloat16) * (size_t)o);
+    if (e == cudaSuccess) e = cudaMalloc(&p->g, f4 + sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc(&p->m, f4);
+    if (e == cudaSuccess) e = cudaMalloc(&p->v, f4);
+    if (e == cudaSuccess) e = cudaMalloc(&tail, fi + sizeof(unsigned));
+    p->tail = tail;
     if (e == cudaSuccess) {
-        p->w = (float*)mem; p->g = (float*)(mem + f4); p->m = (float*)(mem + 2 * f4); p->v = (float*)mem2;
         p->loss = p->g + o;
-        p->wb = (__nv_bfloat16*)(mem2 + f4);
-        p->err = (unsigned*)(mem2 + f4 + f2 + fi);
+        p->err = (unsigned*)(tail + fi);
         if (fused) {
             p->kx = in_dim <= 16 ? 16 : 32;
-            p->img = (__nv_bfloat16*)(mem2 + f4 + f2);
+            p->img = (__nv_bfloat16*)tail;
         }
         // zero moments, error flag and the padded inputs' weights
-        e = cudaMemset(mem + f4, 0, 2 * f4);
-        if (e == cudaSuccess) e = cudaMemset(mem2, 0, f4 + f2 + fi + 256);
+        e = cudaMemset(p->m, 0, f4);
+        if (e == cudaSuccess) e = cudaMemset(p->v, 0, f4);
+        if (e == cudaSuccess) e = cudaMemset(tail, 0, fi + sizeof(unsigned));
     }
     static std::atomic<uint64_t> ready{0};   // devices whose attributes are set
     if (e == cudaSuccess && fused && !((ready.load() >> (device & 63)) & 1)) {
@@ -782,7 +781,7 @@ int dtb_mlp_destroy(dtb_mlp* p)
     cudaGetDevice(&prev);
     cudaSetDevice(p->device);
     if (p->act) { cudaFree(p->act); p->Z1 = p->H1 = p->H2 = p->dZ2 = p->dZ1 = p->dY = nullptr; }
-    void* bufs[] = {p->mem, p->mem2, p->Z1, p->H1, p->Z2, p->H2, p->Y,
+    void* bufs[] = {p->w, p->wb, p->g, p->m, p->v, p->tail, p->Z1, p->H1, p->Z2, p->H2, p->Y,
                     p->dY, p->dH2, p->dZ2, p->dH1, p->dZ1};
     for (void* b : bufs) if (b) cudaFree(b);
     if (prev >= 0) cudaSetDevice(prev);
