@@ -158,7 +158,6 @@ struct dtb_block {
     // pinned host staging
     void* pinned = nullptr;
     size_t pinned_bytes = 0;
-    RunParams* h_run = nullptr;   // pinned
     // auto mode
     int64_t launches = 0;
     uint64_t samples_from = 0;    // step at which sampling started
@@ -553,7 +552,6 @@ static void destroy_block(dtb_block* b)
     for (void* p : b->allocs) cudaFree(p);
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
     if (b->pinned) cudaFreeHost(b->pinned);
-    if (b->h_run) cudaFreeHost(b->h_run);
     delete b;
 }
 
@@ -562,7 +560,6 @@ static int rebuild_groups(dtb_block* b, const int32_t* sub_to_region);
 static int finish_create(dtb_block* b)
 {
     RET(rebuild_groups(b, nullptr));
-    CK(cudaMallocHost((void**)&b->h_run, sizeof(RunParams)));
     RET(ensure_stats(b, 256));
     CK(cudaStreamSynchronize(b->stream));
     return DTB_OK;
@@ -1158,10 +1155,8 @@ static int ensure_method(dtb_block* b, int mm)
 
 static int set_run_params(dtb_block* b, float noise_rate, int isolated)
 {
-    b->h_run->run_base = b->steps;
-    b->h_run->noise_rate = noise_rate;
-    b->h_run->isolated = isolated ? 1 : 0;
-    CK(cudaMemcpyAsync(&b->ds.ctl->run_base, b->h_run, sizeof(RunParams), cudaMemcpyHostToDevice, b->stream));
+    k_set_run<<<1, 1, 0, b->stream>>>(b->ds.ctl, noise_rate, isolated ? 1 : 0);
+    CK(cudaGetLastError());
     return DTB_OK;
 }
 

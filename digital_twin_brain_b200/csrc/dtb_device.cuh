@@ -60,7 +60,7 @@ static_assert(sizeof(ParamClass) == 96, "ParamClass layout");
 // last CTA of each update kernel.
 struct Ctl {
     unsigned long long steps_done;   // number of completed updates (Philox step counter)
-    // per-run parameters, written by the host as one 16-byte copy
+    // per-run parameters (k_set_run)
     unsigned long long run_base;     // steps_done at the start of the current run (stats row 0)
     float noise_rate;                // >= 0: scalar rate; < 0: per-class rate
     int32_t isolated;                // block.run(isolated=...)
@@ -75,13 +75,6 @@ struct Ctl {
                                      // scatter that follows advances
 };
 static_assert(sizeof(Ctl) == 64, "Ctl layout");
-
-struct RunParams {
-    unsigned long long run_base;
-    float noise_rate;
-    int32_t isolated;
-};
-static_assert(sizeof(RunParams) == 16, "RunParams layout");
 
 // Constants of the float64 BOLD step (bold_model_pytorch.py:43-78): reciprocals of the time
 // constants and of E_0, and ln(1 - E_0) in two parts.

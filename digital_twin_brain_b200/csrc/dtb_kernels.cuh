@@ -455,6 +455,17 @@ __device__ __forceinline__ void deferred_stats(const DevState& s)
     }
 }
 
+// The parameters of the steps queued behind it: arguments by value, so that the calls and chunks
+// queued before these steps, and a replay of a caller's graph, each keep their own (a copy from one
+// host buffer would be read when the stream gets there).  Launched outside the step chain: the clock
+// it reads is the last step's.
+__global__ void k_set_run(Ctl* ctl, float noise_rate, int32_t isolated)
+{
+    ctl->run_base = ctl->steps_done;
+    ctl->noise_rate = noise_rate;
+    ctl->isolated = isolated;
+}
+
 // ------------------------------------------------------------ samples
 // cuda/src/stage/sample.cpp:8-26 / stat_result.cpp:283-305: spike and V of the
 // sampled neurons after the step just taken, into a ring of steps.
