@@ -579,15 +579,32 @@ int check_err(dtb_mlp* p)
     return DTB_OK;
 }
 
+// A failure is reported here and cleared: the next call's check is not to find it.
+int alloc_f(float** p, size_t count)
+{
+    const cudaError_t e = cudaMalloc(p, sizeof(float) * count);
+    if (e == cudaSuccess) return DTB_OK;
+    *p = nullptr;
+    cudaGetLastError();
+    return mlp_fail(DTB_ERR_CUDA, "cudaMalloc of %zu bytes: %s", sizeof(float) * count, cudaGetErrorString(e));
+}
+
+// The fused kernels' activation buffers: one allocation, and the pointers into it go with it.
+void free_act(dtb_mlp* p)
+{
+    if (!p->act) return;
+    cudaFree(p->act);
+    p->act = p->Z1 = p->H1 = p->H2 = p->dZ2 = p->dZ1 = p->dY = nullptr;
+    p->cap = 0;
+}
+
 int ensure_cap(dtb_mlp* p, int64_t B)
 {
     if (B <= p->cap) return DTB_OK;
     if (p->img) {   // the fused kernels' buffers, in one allocation
-        if (p->act) cudaFree(p->act);
-        p->act = nullptr;
-        p->cap = 0;
+        free_act(p);
         const size_t n = (size_t)B * p->H;
-        MCK(cudaMalloc(&p->act, sizeof(float) * (5 * n + (size_t)B)));
+        if (int rc = alloc_f(&p->act, 5 * n + (size_t)B)) return rc;
         p->Z1 = p->act; p->H1 = p->Z1 + n; p->H2 = p->H1 + n; p->dZ2 = p->H2 + n; p->dZ1 = p->dZ2 + n;
         p->dY = p->dZ1 + n;
         p->cap = B;
@@ -599,9 +616,10 @@ int ensure_cap(dtb_mlp* p, int64_t B)
     if (p->dY) cudaFree(p->dY);
     p->Y = p->dY = nullptr;
     p->cap = 0;
-    for (float** b : bufs) MCK(cudaMalloc(b, sizeof(float) * (size_t)B * p->H));
-    MCK(cudaMalloc(&p->Y, sizeof(float) * (size_t)B));
-    MCK(cudaMalloc(&p->dY, sizeof(float) * (size_t)B));
+    for (float** b : bufs)
+        if (int rc = alloc_f(b, (size_t)B * p->H)) return rc;
+    if (int rc = alloc_f(&p->Y, (size_t)B)) return rc;
+    if (int rc = alloc_f(&p->dY, (size_t)B)) return rc;
     p->cap = B;
     return DTB_OK;
 }
@@ -780,7 +798,7 @@ int dtb_mlp_destroy(dtb_mlp* p)
     int prev = -1;
     cudaGetDevice(&prev);
     cudaSetDevice(p->device);
-    if (p->act) { cudaFree(p->act); p->Z1 = p->H1 = p->H2 = p->dZ2 = p->dZ1 = p->dY = nullptr; }
+    free_act(p);
     void* bufs[] = {p->w, p->wb, p->g, p->m, p->v, p->tail, p->Z1, p->H1, p->Z2, p->H2, p->Y,
                     p->dY, p->dH2, p->dZ2, p->dH1, p->dZ1};
     for (void* b : bufs) if (b) cudaFree(b);

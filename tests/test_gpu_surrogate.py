@@ -1,10 +1,14 @@
 """Surrogate MLP kernels: forward and gradients against the float64 CPU oracle,
 and training that fits a smooth function."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 from oracle import mlp_oracle
+from digital_twin_brain_b200 import _lib
+from digital_twin_brain_b200._lib import DtbError
 from digital_twin_brain_b200.surrogate import MLP, RateSurrogate
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +69,30 @@ def test_shapes_match_oracle(inputs, hidden, B):
     g, loss = m.gradient(torch.from_numpy(x), torch.from_numpy(t))
     assert abs(loss - loss_ref) <= 1e-4 * loss_ref
     assert np.abs(g.cpu().numpy() - g_ref).max() <= 1e-4 * np.abs(g_ref).max()
+
+
+@pytest.mark.parametrize("hidden", [256, 64])
+def test_failed_growth_leaves_other_owners_alone(hidden):
+    """Activations that cannot grow: the call reports it, the network stays usable, and closing it
+    frees nothing that another network has been given in the meantime."""
+    rng = np.random.default_rng(7)
+    x = torch.from_numpy(rng.normal(0, 1, (360, 14)).astype(np.float32)).cuda()
+    t = torch.from_numpy(rng.normal(0, 1, 360).astype(np.float32)).cuda()
+    a = MLP(14, hidden, seed=5, device=0)
+    want, loss = a.gradient(x, t)
+    with pytest.raises(DtbError):      # 2^40 rows: refused by the allocation, before anything is launched
+        _lib.call("dtb_mlp_gradient", a._h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(t.data_ptr()), 1 << 40,
+                  None, None)
+    b = MLP(14, hidden, seed=5, device=0)
+    b.gradient(x, t)                   # the same sizes: the memory a gave back
+    a.close()
+    g, again = b.gradient(x, t)
+    # the gradient's partial sums meet in any order
+    np.testing.assert_allclose(g.cpu().numpy(), want.cpu().numpy(), rtol=1e-4, atol=1e-5 * float(want.abs().max()))
+    assert abs(again - loss) <= 1e-5 * loss
+    c = MLP(14, hidden, seed=5, device=0)
+    with pytest.raises(DtbError):
+        _lib.call("dtb_mlp_gradient", c._h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(t.data_ptr()), 1 << 40,
+                  None, None)
+    assert abs(c.gradient(x, t)[1] - loss) <= 1e-5 * loss
+    c.close()
