@@ -594,9 +594,9 @@ static int rebuild_groups(dtb_block* b, const int32_t* sub_to_region)
         for (int i = 0; i <= n_sub; ++i) ptr.push_back(i);
         for (int i = 0; i < n_sub; ++i) { sub.push_back(i); reg.push_back(-1); }
     }
-    CK(cudaStreamSynchronize(b->stream));   // the previous tables are no longer in use
-    dfree(b, s.grp_ptr);
-    std::vector<int32_t> all(ptr);           // one table: pointers, subblocks, regions
+    // One table: pointers, subblocks, regions.  The previous one is kept until the handle goes: runs in
+    // a CUDA graph of the caller's may still read it.
+    std::vector<int32_t> all(ptr);
     all.insert(all.end(), sub.begin(), sub.end());
     all.insert(all.end(), reg.begin(), reg.end());
     int32_t* dp = nullptr;
@@ -2441,11 +2441,10 @@ int dtb_block_update_property(dtb_block* b, const float* property, const float* 
     CK(cudaMemcpy(const_cast<uint32_t*>(s.cls), cls.data(), sizeof(uint32_t) * (size_t)b->N, cudaMemcpyHostToDevice));
     RET(upload_tile_classes(b, cls));
     if (!s.st_spk) RET(ensure_stats(b, 256));
-    if (b->bold_R == 0) RET(rebuild_groups(b, nullptr));
+    if (b->bold_R == 0 && b->grp_n_sub != b->n_sub) RET(rebuild_groups(b, nullptr));
     b->class_prop_base.clear();
     s.gnrn = nullptr;   // the new matrix holds every neuron's g_ui: gamma factors no longer apply
     drop_graphs(b);     // captured graphs hold the update's form for the old gnrn
-    drop_graphs(b);
     b->override_pending = true;
     return DTB_OK;
 }

@@ -67,3 +67,31 @@ def test_captured_run_replays_with_its_own_arguments():
                                       b.run(7, noise_rate=0.3, isolated=True, mode="push")[2])
         x, y = (net.run(5, noise_rate=0.02, isolated=True, mode="push")[2] for net in (a, b))
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("N", [2000, 20000])     # one cluster launch; a chain of per-step kernels
+def test_captured_run_outlives_new_statistics_tables(N):
+    """The statistics tables that a captured run reads stay readable after BOLD is attached again."""
+    spec = synthetic.single_block(N, 20, gen_seed=1)
+    a, b = (Network.from_spec(spec, device=0) for _ in range(2))
+    side = torch.cuda.Stream()
+    a.set_stream(side)
+    for net in (a, b):
+        net.run(32, noise_rate=0.01, isolated=True, mode="push")
+    out = (torch.empty((7, a.n_sub), device="cuda"), torch.empty((7, a.n_sub), device="cuda"),
+           torch.empty((7,), dtype=torch.int32, device="cuda"))
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=side):
+        _run(a, 7, 0.3, out)
+    held = [a.info().device_bytes]
+    for _ in range(3):
+        a.attach_bold(spec.sub_to_region(), spec.R)
+        held.append(a.info().device_bytes)
+        filler = [torch.full((64,), -1, dtype=torch.int32, device="cuda") for _ in range(64)]   # what was given back is used
+        g.replay()
+        torch.cuda.synchronize()
+        del filler
+        np.testing.assert_array_equal(out[2].cpu().numpy().view(np.uint32),
+                                      b.run(7, noise_rate=0.3, isolated=True, mode="push")[2])
+    assert held[-1] - held[-2] <= 4096     # a few small tables a time
