@@ -110,6 +110,7 @@ _SIGS = {
     "dtb_mlp_forward": [c_vp, c_vp, c_i64, c_vp],
     "dtb_mlp_gradient": [c_vp, c_vp, c_vp, c_i64, c_vp, c_vp],
     "dtb_mlp_train_step": [c_vp, c_vp, c_vp, c_i64, c_f32, c_vp],
+    "dtb_mlp_set_wait_limit": [c_vp, c_u32],
     "dtb_mlp_last_error": [c_char_p, c_size_t],
 }
 

@@ -463,16 +463,19 @@ __global__ void k_colsum(int64_t rows, int cols, const float* __restrict__ dZ, f
 
 // Adam on the FP32 master weights; refresh the BF16 compute copy (and the fused kernels' images of it).
 __global__ void k_adam(int64_t n, float* w, const float* __restrict__ g, float* m, float* v, __nv_bfloat16* wb,
-                       float lr, float b1, float b2, float eps, float c1, float c2, __nv_bfloat16* img, int in, int kx)
+                       float lr, float b1, float b2, float eps, float c1, float c2, __nv_bfloat16* img, int in, int kx,
+                       const unsigned* err)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float gi = g[i];
+    const unsigned bad = *err;
+    const float gi = g[i], w0 = w[i];
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+    const float wi = w0 - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    if (bad) return;   // a pass that gave up left no gradient: weights and moments stay
     m[i] = mi;
     v[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     w[i] = wi;
     const __nv_bfloat16 h = __float2bfloat16_rn(wi);
     wb[i] = h;
@@ -512,6 +515,7 @@ struct dtb_mlp {
     float *dY = nullptr, *dH2 = nullptr, *dZ2 = nullptr, *dH1 = nullptr, *dZ1 = nullptr;
     int64_t t = 0;                 // Adam step
     unsigned* err = nullptr;       // device flag: a tensor-core GEMM gave up waiting for its MMAs
+    uint32_t wait_limit = kNetWait;   // polls of the fused kernels' waits
 };
 
 namespace {
@@ -634,7 +638,7 @@ int net_pass(dtb_mlp* p, const float* x, const float* target, int64_t B, float* 
     g.img2 = p->img; g.img2t = p->img + kNetImgW2; g.img1 = p->img + 2 * kNetImgW2;
     g.b1 = p->w + p->o_b1; g.b2 = p->w + p->o_b2; g.b3 = p->w + p->o_b3;
     g.w3 = p->wb + p->o_W3;
-    g.y = y; g.err = p->err;
+    g.y = y; g.err = p->err; g.wait = p->wait_limit;
     // the most copies of a row that still fit one CTA per SM in one wave
     const int D = cdiv(B, kNetRows / 4) <= kNetSMs ? 4 : (cdiv(B, kNetRows / 2) <= kNetSMs ? 2 : 1);
     const unsigned grid = cdiv(B, kNetRows / D);
@@ -664,7 +668,7 @@ int net_gradient(dtb_mlp* p, const float* x, const float* target, int64_t B)
     a.x = x; a.H1 = p->H1; a.H2 = p->H2; a.dZ2 = p->dZ2; a.dZ1 = p->dZ1; a.dY = p->dY;
     a.gW1 = p->g + p->o_W1; a.gb1 = p->g + p->o_b1; a.gW2 = p->g + p->o_W2; a.gb2 = p->g + p->o_b2;
     a.gW3 = p->g + p->o_W3; a.gb3 = p->g + p->o_b3;
-    a.err = p->err;
+    a.loss = p->loss; a.err = p->err; a.wait = p->wait_limit;
     k_net_grad<<<dim3(2, cdiv(B, a.rows_per_split)), kNetThreads, kGradSmem, p->stream>>>(a);
     MCK(cudaGetLastError());
     return DTB_OK;
@@ -814,6 +818,13 @@ int dtb_mlp_set_stream(dtb_mlp* p, void* stream)
     return DTB_OK;
 }
 
+int dtb_mlp_set_wait_limit(dtb_mlp* p, uint32_t polls)
+{
+    if (!p) return mlp_fail(DTB_ERR_ARG, "null handle");
+    p->wait_limit = polls;
+    return DTB_OK;
+}
+
 int dtb_mlp_n_params(const dtb_mlp* p, int64_t* n)
 {
     if (!p || !n) return mlp_fail(DTB_ERR_ARG, "null argument");
@@ -871,7 +882,7 @@ int dtb_mlp_train_step(dtb_mlp* p, const float* x, const float* target, int64_t 
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f - std::pow(b1, (float)p->t), c2 = 1.0f - std::pow(b2, (float)p->t);
     k_adam<<<cdiv(p->n_params, 256), 256, 0, p->stream>>>(p->n_params, p->w, p->g, p->m, p->v, p->wb, lr, b1, b2,
-                                                          1e-8f, c1, c2, p->img, p->in, p->kx);
+                                                          1e-8f, c1, c2, p->img, p->in, p->kx, p->err);
     MCK(cudaGetLastError());
     return DTB_OK;
 }

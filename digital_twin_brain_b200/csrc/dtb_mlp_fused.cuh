@@ -29,7 +29,8 @@ constexpr int kNetTermBytes = kNetRows * kNetChunk * 2;           // one BF16 te
 constexpr int kNetW2Bytes = kNetH * kNetH * 2;
 constexpr int kNetImgW2 = kNetH * kNetH;                           // elements
 constexpr int kNetTmemCols = 512;
-constexpr uint32_t kNetWait = 1u << 22;
+constexpr uint32_t kNetWait = 1u << 22;   // polls of a wait before it is given up (dtb_mlp_set_wait_limit)
+constexpr uint32_t kNetDrain = 1u << 24;  // ... of the copies and MMAs still in flight at the end
 
 // Element (row, k) of a K-major operand image of R rows: core matrices of 8 rows x 8 k (128 bytes),
 // row groups adjacent, K groups R / 8 core matrices apart.
@@ -137,6 +138,7 @@ struct NetArgs {
     float *Z1, *H1, *H2, *dZ2, *dZ1, *dY;  // [B][256] (training), dY [B]
     float* loss;
     unsigned* err;
+    uint32_t wait;                         // polls of a wait before it is given up
 };
 
 constexpr int kNetOffA = kNetW2Bytes;                               // the chunk's three terms
@@ -151,6 +153,9 @@ static_assert(kNetSmem <= 227 * 1024, "shared memory of one CTA");
 // the D quadrants share a row's columns, so that a batch too small to fill the GPU with 128-row tiles
 // spends 1 / D of the time on the elementwise work that bounds it (gradient of 4,096 rows 124 -> 87 us,
 // Adam step on 360 rows 92 -> 54 us against D = 1).
+// A thread whose wait is given up on stores nothing from then on, nor does any other after the next
+// barrier, where no further MMAs are issued either: y of the CTA's rows and the loss become NaN, and
+// the error flag keeps the weight gradients and Adam from using what was not computed.
 template <bool TRAIN, int D>
 __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
 {
@@ -210,29 +215,32 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
     const uint32_t tlane = tmem + ((uint32_t)(quad * 32) << 16);
     const uint32_t idesc = mma_idesc(kNetH);
     bool ok = true;
-    if (tid == 0) {   // layer 1: Z1 = X W1^T
-        ok = mma_wait(b_w1, 0, kNetWait);
+    bool l1 = false, w2t = false;   // thread 0: committed to b_l1; copy of W2^T issued
+    int n_ch = 0;                   // thread 0: commits to b_ch
+    if (tid == 0 && (ok = mma_wait(b_w1, 0, g.wait))) {   // layer 1: Z1 = X W1^T
         for (int s = 0; s < g.kx / 16; ++s)
             for (int i = 0; i < 3; ++i)
                 net_mma(tmem, net_desc(smem_addr(sX + i * xterm + s * 2 * (kNetRows / 8) * 128), (kNetRows / 8) * 128, 128),
                         net_desc(smem_addr(sW1 + s * 2 * (kNetH / 8) * 128), (kNetH / 8) * 128, 128), idesc, s + i > 0);
         net_commit(b_l1);
+        l1 = true;
     }
-    ok = mma_wait(b_l1, 0, kNetWait) && ok;
+    ok = ok && mma_wait(b_l1, 0, g.wait);
+    __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     // One operand chunk: the thread's kCols values of chunk q's columns into the buffer once the MMAs
     // that read the chunk before are done, then this chunk's MMAs into accumulator columns d (first: q == q0).
     auto chunk = [&](int q, int q0, uint32_t d, const float* v) {
-        if (q >= 1) ok = mma_wait(b_ch, (uint32_t)((q - 1) & 1), kNetWait) && ok;
+        if (q >= 1) ok = ok && mma_wait(b_ch, (uint32_t)((q - 1) & 1), g.wait);
 #pragma unroll
         for (int c = 0; c < kCols / 8; ++c)
             net_split8(v + c * 8, sA + ((grp * (kCols / 8) + c) * (kNetRows / 8) + (r >> 3)) * 128 + (r & 7) * 16, kNetTermBytes,
                        D, kRows * 16);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
+        ok = __syncthreads_and(ok);
+        if (tid == 0 && ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int k8 = (q - q0) * (kNetChunk / 8);
             for (int s = 0; s < kNetChunk / 16; ++s)
@@ -241,26 +249,31 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
                             net_desc(smem_addr(sW2 + (k8 + 2 * s) * (kNetH / 8) * 128), (kNetH / 8) * 128, 128), idesc,
                             q > q0 || s + i > 0);
             net_commit(b_ch);
+            ++n_ch;
         }
     };
 
     // ---- layer 2: Z2 = GELU(Z1 + b1) W2^T, chunk by chunk
-    if (tid == 0) ok = mma_wait(b_w2, 0, kNetWait) && ok;
+    if (tid == 0) ok = ok && mma_wait(b_w2, 0, g.wait);
     for (int q = 0; q < kNetChunks; ++q) {
         float v[kCols];
         const int c0 = q * kNetChunk + grp * kCols;
         net_ld<kCols>(tlane + (uint32_t)c0, v);
 #pragma unroll
         for (int e = 0; e < kCols; ++e) v[e] += sb1[c0 + e];
-        if (TRAIN && live) net_store<kCols>(g.Z1 + row * kNetH + c0, v);
+        if (TRAIN && live && ok) net_store<kCols>(g.Z1 + row * kNetH + c0, v);
 #pragma unroll
         for (int e = 0; e < kCols; ++e) v[e] = gelu(v[e]);
-        if (TRAIN && live) net_store<kCols>(g.H1 + row * kNetH + c0, v);
+        if (TRAIN && live && ok) net_store<kCols>(g.H1 + row * kNetH + c0, v);
         chunk(q, 0, tmem + kNetH, v);
     }
-    ok = mma_wait(b_ch, (uint32_t)((kNetChunks - 1) & 1), kNetWait) && ok;
+    ok = ok && mma_wait(b_ch, (uint32_t)((kNetChunks - 1) & 1), g.wait);
+    __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (TRAIN && tid == 0) net_bulk(smem_addr(sW2), g.img2t, (uint32_t)kNetW2Bytes, b_w2);   // every MMA that read W2 is done
+    if (TRAIN && tid == 0 && ok) {
+        net_bulk(smem_addr(sW2), g.img2t, (uint32_t)kNetW2Bytes, b_w2);   // every MMA that read W2 is done
+        w2t = true;
+    }
 
     // ---- output: y = GELU(Z2 + b2) . w3 + b3
     float p = 0.0f;
@@ -273,13 +286,15 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
             v[e] = gelu(v[e] + sb2[c0 + e]);
             p = fmaf(v[e], sw3[c0 + e], p);
         }
-        if (TRAIN && live) net_store<kCols>(g.H2 + row * kNetH + c0, v);
+        if (TRAIN && live && ok) net_store<kCols>(g.H2 + row * kNetH + c0, v);
     }
     sy[grp * kRows + r] = p;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    ok = __syncthreads_and(ok);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (tid < kRows) {   // threads 0 .. kRows - 1: tile row tid (grp 0 of the first quadrants)
+    if (tid < kRows && !ok) {
+        if (live && g.y) g.y[row] = nanf("");
+    } else if (tid < kRows) {   // threads 0 .. kRows - 1: tile row tid (grp 0 of the first quadrants)
         float y = sy[tid];
 #pragma unroll
         for (int i = 1; i < 2 * D; ++i) y += sy[i * kRows + tid];
@@ -300,23 +315,24 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
         __syncthreads();
         const float dy = sdy[r];
         // ---- dZ2 = dy w3 GELU'(Z2), and dH1 = dZ2 W2 over Z1's accumulator columns
-        if (tid == 0) ok = mma_wait(b_w2, 1, kNetWait) && ok;
+        if (tid == 0) ok = ok && mma_wait(b_w2, 1, g.wait);
         for (int q = kNetChunks; q < 2 * kNetChunks; ++q) {
             float v[kCols];
             const int c0 = (q - kNetChunks) * kNetChunk + grp * kCols;
             net_ld<kCols>(tlane + (uint32_t)(kNetH + c0), v);
 #pragma unroll
             for (int e = 0; e < kCols; ++e) v[e] = (dy * sw3[c0 + e]) * gelu_grad(v[e] + sb2[c0 + e]);
-            if (live) net_store<kCols>(g.dZ2 + row * kNetH + c0, v);
+            if (live && ok) net_store<kCols>(g.dZ2 + row * kNetH + c0, v);
             chunk(q, kNetChunks, tmem, v);
         }
-        ok = mma_wait(b_ch, (uint32_t)((2 * kNetChunks - 1) & 1), kNetWait) && ok;
+        ok = ok && mma_wait(b_ch, (uint32_t)((2 * kNetChunks - 1) & 1), g.wait);
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int q = 0; q < kNetChunks; ++q) {   // dZ1 = dH1 GELU'(Z1), Z1 as this thread wrote it above
             float v[kCols];
             const int c0 = q * kNetChunk + grp * kCols;
             net_ld<kCols>(tlane + (uint32_t)c0, v);
-            if (live) {
+            if (live && ok) {
                 const float4* z1 = reinterpret_cast<const float4*>(g.Z1 + row * kNetH + c0);
 #pragma unroll
                 for (int e = 0; e < kCols; e += 4) {
@@ -328,14 +344,19 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
             }
         }
     }
-    if (!ok) {   // a wait was given up on: flag it, and let copies and MMAs in flight land before shared memory and TMEM go
-        if (g.err) atomicOr(g.err, 1u);
-        mma_wait(b_w1, 0, 1u << 24);
-        mma_wait(b_w2, TRAIN ? 1u : 0u, 1u << 24);
-        mma_wait(b_ch, (uint32_t)(((TRAIN ? 2 : 1) * kNetChunks - 1) & 1), 1u << 24);
-    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    ok = __syncthreads_and(ok);
+    if (!ok) {   // a wait was given up on: flag it, and let copies and MMAs in flight land before shared memory and TMEM go
+        if (tid == 0) {
+            if (g.err) atomicOr(g.err, 1u);
+            if (TRAIN) atomicAdd(g.loss, nanf(""));
+            mma_wait(b_w1, 0, kNetDrain);
+            mma_wait(b_w2, w2t ? 1u : 0u, kNetDrain);
+            if (l1) mma_wait(b_l1, 0, kNetDrain);
+            if (n_ch) mma_wait(b_ch, (uint32_t)((n_ch - 1) & 1), kNetDrain);
+        }
+        __syncthreads();
+    }
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"((uint32_t)kNetTmemCols)
@@ -364,7 +385,9 @@ struct GradArgs {
     int64_t B, rows_per_split;
     const float *x, *H1, *H2, *dZ2, *dZ1, *dY;
     float *gW1, *gb1, *gW2, *gb2, *gW3, *gb3;
+    float* loss;
     unsigned* err;
+    uint32_t wait;
 };
 
 __global__ void __launch_bounds__(kNetThreads, 1) k_net_grad(GradArgs g)
@@ -393,9 +416,9 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_grad(GradArgs g)
     const uint32_t tmem = tmem_base;
     float s_b2 = 0.0f, s_b1 = 0.0f, s_w3 = 0.0f, s_b3 = 0.0f;
     bool ok = true;
-    int st = 0;
+    int st = 0, n_st = 0;   // stages; thread 0: those whose MMAs were issued
     for (int64_t r0 = r_begin; r0 < r_end; r0 += kGradStage, ++st) {
-        if (st > 0) ok = mma_wait(mb, (uint32_t)((st - 1) & 1), kNetWait) && ok;   // the operands are free again
+        if (st > 0) ok = ok && mma_wait(mb, (uint32_t)((st - 1) & 1), g.wait);   // the operands are free again
         // H1^T: thread = column i, eight row groups
 #pragma unroll 4
         for (int c = 0; c < kGradStage / 8; ++c) {
@@ -442,8 +465,8 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_grad(GradArgs g)
             net_split8(v, gsm + kGradOffX + (c * (g.kx / 8) + (f >> 3)) * 128 + (f & 7) * 16, kGradX);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
+        ok = __syncthreads_and(ok);
+        if (tid == 0 && ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int s = 0; s < kGradStage / 16; ++s)
                 for (int i = 0; i < 3; ++i)
@@ -457,14 +480,18 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_grad(GradArgs g)
                                          (uint32_t)(g.kx / 8) * 128, 128), mma_idesc(g.kx), acc);
                     }
             net_commit(mb);
+            ++n_st;
         }
     }
-    if (st > 0) {
-        ok = mma_wait(mb, (uint32_t)((st - 1) & 1), kNetWait) && ok;
-        if (!ok) {
-            if (g.err) atomicOr(g.err, 1u);
-            mma_wait(mb, (uint32_t)((st - 1) & 1), 1u << 24);
-        }
+    const unsigned earlier = tid == 0 ? __ldcg(g.err) : 0u;   // a pass before gave up: there is nothing to add
+    if (st > 0) ok = ok && mma_wait(mb, (uint32_t)((st - 1) & 1), g.wait);
+    ok = __syncthreads_and(ok && earlier == 0u);
+    if (!ok && tid == 0) {   // a wait was given up on: nothing is added, and MMAs in flight end before TMEM goes
+        atomicOr(g.err, 1u);
+        atomicAdd(g.loss, nanf(""));
+        if (n_st) mma_wait(mb, (uint32_t)((n_st - 1) & 1), kNetDrain);
+    }
+    if (st > 0 && ok) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // thread: output row 128 x + 32 (w % 4) + lane, 128 of the 256 columns
         const int m = blockIdx.x * 128 + (warp & 3) * 32 + lane;

@@ -96,3 +96,33 @@ def test_failed_growth_leaves_other_owners_alone(hidden):
                   None, None)
     assert abs(c.gradient(x, t)[1] - loss) <= 1e-5 * loss
     c.close()
+
+
+@pytest.mark.parametrize("B", [1, 300, 5000, 9500])     # four, two and one copy of a row in the tile
+@pytest.mark.parametrize("limit", [0, 1, 2])            # polls: none of the waits, or some, are given up
+def test_given_up_waits_yield_no_results(B, limit):
+    rng = np.random.default_rng(B)
+    x = torch.from_numpy(rng.normal(0, 1, (B, 14)).astype(np.float32)).cuda()
+    t = torch.from_numpy(rng.normal(0, 1, B).astype(np.float32)).cuda()
+    m = MLP(14, 256, seed=5, device=0)
+    w, y = m.params(), m.forward(x).cpu().numpy()
+    _lib.call("dtb_mlp_set_wait_limit", m._h, limit)
+    z = m.forward(x).cpu().numpy()
+    lost = np.isnan(z)
+    np.testing.assert_array_equal(z[~lost], y[~lost])
+    g, loss = m.gradient(x, t)
+    if limit == 0:
+        assert lost.all() and np.isnan(loss) and float(g.abs().max()) == 0.0
+    given_up = bool(lost.any()) or np.isnan(loss)
+    if given_up:
+        _lib.call("dtb_mlp_set_wait_limit", m._h, 1 << 22)
+        assert np.isnan(m.gradient(x, t)[1])            # not reported yet
+        m.train_step(x, t, 1e-2)
+        with pytest.raises(DtbError):
+            m.params()
+        np.testing.assert_array_equal(m.params(), w)    # reported once; the step changed nothing
+    _lib.call("dtb_mlp_set_wait_limit", m._h, 1 << 22)
+    np.testing.assert_array_equal(m.forward(x).cpu().numpy(), y)
+    assert np.isfinite(m.gradient(x, t)[1])
+    m.train_step(x, t, 1e-2)
+    assert (m.params() != w).any()
