@@ -163,6 +163,8 @@ struct dtb_block {
     uint64_t samples_from = 0;    // step at which sampling started
     int64_t samples_written = 0;
     double last_frac = -1.0;
+    double class_noise = 0.0;     // mean of the classes' own noise rates
+    double seen_spikes = -1.0;    // fraction propagating beyond the noise in the latest run whose counts the host saw
     double pull_threshold = 0.05;
     int chunk = 32;
     int scatter_wpw = 0;          // bitmask words per warp in the push scatter (0: by network size)
@@ -392,10 +394,18 @@ static int alloc_state(dtb_block* b)
     return DTB_OK;
 }
 
+static void note_class_noise(dtb_block* b)
+{
+    double sum = 0.0;
+    for (const ParamClass& p : b->classes) sum += p.noise > 0.0f ? std::min(1.0, (double)p.noise) : 0.0;
+    b->class_noise = b->classes.empty() ? 0.0 : sum / (double)b->classes.size();
+}
+
 // Class table, per-neuron class ids, subblock tables and initial V.
 static int upload_class_tables(dtb_block* b)
 {
     DevState& s = b->ds;
+    note_class_noise(b);
     if (b->n_classes > b->pc_cap || !b->d_pc) {
         const int cap = std::max(64, b->n_classes);
         RET(dalloc(b, &b->d_pc, (size_t)cap));
@@ -1212,9 +1222,42 @@ static int emit_stats(dtb_block* b, int rows, int64_t row0, float* sum_out, floa
     return DTB_OK;
 }
 
-// CTAs of the small-network step loop (k_small) for a run of method `method`, or 0 when the
-// per-step kernels serve it.
-static int small_ctas(const dtb_block* b, int method)
+// The fraction of neurons that a run's steps are expected to propagate: the noise of the call plus
+// what earlier runs showed beyond theirs (spikes); before any did, 1 % of the neurons.
+static double noise_of(const dtb_block* b, float noise_rate)
+{
+    return noise_rate >= 0.0f ? std::min(1.0, (double)noise_rate) : b->class_noise;
+}
+
+static double expected_activity(const dtb_block* b, float noise_rate, int isolated)
+{
+    const double noise = noise_of(b, noise_rate);
+    if (isolated) return noise;
+    return std::min(1.0, noise + (b->seen_spikes >= 0.0 ? b->seen_spikes : 0.01));
+}
+
+// Whether the loop is the better one for `f` of the neurons propagating a step.  A neuron holds `cap`
+// contributions; a row that gets more is gathered whole by one of the few warps (a step of 12,288
+// neurons, K = 1000: 35 us at 2 contributions a neuron, 1257 at 10), and 8 of 148 SMs take the events.
+// Push, loop / step kernels, us a step: N = 2,000, K = 1000: 13 / 14 at p = 0.002, 29 / 18 at 0.01,
+// 159 / 21 at 0.02; N = 6,000, K = 300: 21 / 14 at 0.01, 39 / 15 at 0.02; N = 12,288, K = 100: 9 / 12
+// at 0.002, 15 / 12 at 0.01, 23 / 13 at 0.02, 63 / 14 at 0.05.  The loop adds in pull order, which the
+// reductions of the step kernels cannot, so the line lies where its time gets out of hand (about half
+// of the capacity, 32,768 events a step) and not at the crossover (about 6,000 events a step).
+// Pull, the same: the step kernels' slots overflow into a gather too (at 12), so the loop is the faster
+// at any activity while it holds as many (N = 6,000, K = 300, p = 0.05: 120 / 510; N = 9,000, K = 1000,
+// p = 0.02: 1707 / 1898); with fewer it is behind from about a quarter of its capacity on (N = 12,288,
+// K = 100: 16 / 17 at p = 0.01, 24 / 23 at 0.02, 64 / 34 at 0.05; K = 1000: 1299 / 545 at 0.01).
+static bool small_pays(const dtb_block* b, int method, int cap, double f)
+{
+    const double events = (double)b->S * f, each = events / (double)b->N;
+    if (method == DTB_MODE_PUSH) return each <= 0.55 * cap && events <= 32768.0;
+    return cap >= (int)kSlotCap || each <= 0.25 * cap;
+}
+
+// CTAs of the small-network step loop (k_small) for a run of method `method` with `f` of the neurons
+// propagating a step, or 0 when the per-step kernels serve it.
+static int small_ctas(const dtb_block* b, int method, double f)
 {
     const DevState& s = b->ds;
     if (b->N <= 0 || b->N > kSmallMaxNeurons) return 0;
@@ -1227,7 +1270,8 @@ static int small_ctas(const dtb_block* b, int method)
     if (b->S > 0x7fffffffLL) return 0;                                   // 32-bit synapse offsets
     const int nt = (int)((b->N + kWarpNeurons - 1) / kWarpNeurons);
     int ctas = (nt + kSmallTilesFew - 1) / kSmallTilesFew;
-    return ctas < kSmallClusterMax ? ctas : kSmallClusterMax;
+    ctas = ctas < kSmallClusterMax ? ctas : kSmallClusterMax;
+    return small_pays(b, method, small_cap((nt + ctas - 1) / ctas), f) ? ctas : 0;
 }
 
 // n steps of k_small and their statistics (rows row0.. of the outputs).  Device outputs are written
@@ -1917,7 +1961,7 @@ int dtb_block_run(dtb_block* b, int n_steps, float noise_rate, int isolated, int
         const int m = choose_mode(b, mode);
         const int mm = resolve_method(b, m);
         const uint32_t cap = b->stats_cap;
-        const int small = small_ctas(b, mm);
+        const int small = small_ctas(b, mm, expected_activity(b, noise_rate, isolated));
         if (!small) RET(ensure_method(b, mm));
         int n;
         if (small > 0) {
@@ -1930,20 +1974,23 @@ int dtb_block_run(dtb_block* b, int n_steps, float noise_rate, int isolated, int
         }
         std::vector<uint32_t> nact;
         const bool want_nact = (mode == DTB_MODE_AUTO) || (m == DTB_MODE_PULL && b->has_qpos && b->pull_method == 0);
+        // (host outputs bring the counts along)
+        std::vector<uint32_t>* const counts = want_nact || where == DTB_HOST ? &nact : nullptr;
         if (small > 0) {
             b->steps += (uint64_t)n;
-            RET(run_small(b, small, n, noise_rate, isolated, done, sum_out, mean_out, nact_out, where,
-                          want_nact ? &nact : nullptr));
+            RET(run_small(b, small, n, noise_rate, isolated, done, sum_out, mean_out, nact_out, where, counts));
         } else {
             RET(set_run_params(b, noise_rate, isolated));
             RET(enqueue_chunk(b, n, mm));
             b->steps += (uint64_t)n;
-            RET(emit_stats(b, n, done, sum_out, mean_out, nact_out, where, want_nact ? &nact : nullptr));
+            RET(emit_stats(b, n, done, sum_out, mean_out, nact_out, where, counts));
         }
-        if (want_nact && n > 0) {
+        if (counts && n > 0) {
             double tot = 0.0;
             for (uint32_t v : nact) tot += v;
-            b->last_frac = tot / ((double)n * (double)std::max<int64_t>(1, b->N));
+            const double frac = tot / ((double)n * (double)std::max<int64_t>(1, b->N));
+            if (want_nact) b->last_frac = frac;
+            if (!isolated) b->seen_spikes = std::max(0.0, frac - noise_of(b, noise_rate));
         }
         done += n;
     }
@@ -2468,6 +2515,7 @@ static int rebuild_dirty_classes(dtb_block* b, const std::vector<char>& dirty,
         p.member = b->classes[(size_t)c].member;
         b->classes[(size_t)c] = p;
     }
+    note_class_noise(b);
     CK(cudaMemcpyAsync(const_cast<ParamClass*>(b->ds.pc), b->classes.data(), sizeof(ParamClass) * b->classes.size(),
                        cudaMemcpyHostToDevice, b->stream));
     CK(cudaStreamSynchronize(b->stream));

@@ -13,6 +13,8 @@
 // The only memory a step waits for is one read of the firing rows' synapses.  The barrier is the
 // hardware cluster barrier (__syncthreads for one CTA): nothing spins.
 // Both propagation modes run this way: the ordered sums are a valid order for push.
+// Runs whose neurons get more contributions a step than their slots hold stay with the per-step
+// kernels (small_pays).
 // Measured (single block of 2,000 neurons, K = 100, p = 0.01): a step of a closed loop 39.9 -> 5.9 us,
 // one step per call with its statistics on the host 87 -> 36 us.  The same loop on a grid of all SMs
 // (counts, slots and J in L2, a barrier in memory) was no faster than two launches a step from

@@ -56,3 +56,48 @@ def test_small_loop_mixed_classes_members_bold_samples():
     for x, y in zip(nets[0].get_samples(), nets[1].get_samples()):
         np.testing.assert_array_equal(x, y)
     np.testing.assert_array_equal(nets[0].window_spikes(), nets[1].window_spikes())
+
+
+@pytest.mark.parametrize("N,K,rate,mode,loop", [
+    (2000, 100, 0.01, "push", True), (2200, 1000, 0.002, "push", True), (2200, 1000, 0.05, "push", False),
+    (2200, 1000, 0.02, "pull", True), (9216, 300, 0.02, "push", False), (9216, 300, 0.05, "pull", True),
+    (9217, 300, 0.05, "pull", False), (12288, 20, 0.05, "push", True), (12288, 20, 0.05, "pull", True),
+    (12288, 100, 0.05, "push", False), (12288, 100, 0.05, "pull", False), (12288, 300, 0.02, "auto", False)])
+def test_loop_serves_what_its_slots_hold(N, K, rate, mode, loop):
+    """One launch for the steps, or two a step, by the contributions a neuron is expected to get; the
+    results are the same either way (pull), or to rounding (push, whose reductions have no order)."""
+    spec = synthetic.single_block(N, K, gen_seed=K, g_ui=tuple(g * 10.0 / K for g in synthetic.LIF["g_ui"]))
+    a, b = (Network.from_spec(spec, device=0) for _ in range(2))
+    b.set_tuning(TUNE_PULL_METHOD, ROWS)
+    # refractory from the start: the noise alone propagates
+    before = a.info().kernel_launches
+    sa, ma, na = a.run(20, noise_rate=rate, mode=mode)
+    launches = a.info().kernel_launches - before
+    assert launches == 1 if loop else launches >= 40
+    sb, mb, nb = b.run(20, noise_rate=rate, mode="pull")
+    np.testing.assert_array_equal(na, nb)
+    np.testing.assert_array_equal(sa, sb)
+    if loop or mode == "pull":
+        _same(a, b)
+        np.testing.assert_array_equal(ma, mb)
+    else:
+        # 20 steps of up to ~30 additions in another order: 600 float32 roundings at most
+        np.testing.assert_allclose(a.get(FIELD_J), b.get(FIELD_J), rtol=4e-5, atol=1e-5)
+        np.testing.assert_allclose(ma, mb, rtol=1e-5)
+
+
+def test_loop_follows_the_activity_seen():
+    """A push run that shows more activity than its noise moves the next runs to the step kernels."""
+    spec = synthetic.single_block(12288, 100, gen_seed=2, I_extern_Input=8.0, T_ref=0.5,
+                                  g_ui=tuple(g * 0.01 for g in synthetic.LIF["g_ui"]))
+    net = Network.from_spec(spec, device=0)
+
+    def launches(n, isolated=False):
+        before = net.info().kernel_launches
+        _, _, na = net.run(n, noise_rate=0.0, isolated=isolated, mode="push")
+        return net.info().kernel_launches - before, na.mean() / net.N
+    first, _ = launches(300)                     # driven over threshold every dozen steps
+    quiet, _ = launches(20, isolated=True)       # noise alone propagates: the loop again
+    driven, f = launches(40)
+    assert f > 0.04 and first < 2 * 300
+    assert quiet == 1 and driven >= 80
