@@ -195,6 +195,7 @@ struct dtb_block {
     uint32_t* d_nact2 = nullptr;
     double* d_vsum2 = nullptr;
     uint32_t* d_unmapped2 = nullptr;
+    int small_fit = -1;           // the device can place its cluster (-1: not asked yet)
     int grp_n_sub = -1;           // subblocks when the statistics groups were built
     bool knobs_set = false;       // the caller chose a schedule (dtb_block_set_tuning): launch per step as asked
     bool chunk_set = false;
@@ -1274,6 +1275,40 @@ static int small_ctas(const dtb_block* b, int method, double f)
     return small_pays(b, method, small_cap((nt + ctas - 1) / ctas), f) ? ctas : 0;
 }
 
+// The launch of k_small: one cluster.  `at`: the configuration's attribute.
+static cudaLaunchConfig_t small_config(const dtb_block* b, int ctas, cudaLaunchAttribute* at)
+{
+    const int nt = (int)((b->N + kWarpNeurons - 1) / kWarpNeurons), tiles = (nt + ctas - 1) / ctas;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = small_smem(tiles, small_cap(tiles));
+    cfg.stream = b->stream;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Whether the device can place that cluster: its CTAs take an SM each, in one GPC, with up to 224 KB
+// of shared memory, which a partition of the device may not have.  (Asked once: a network's cluster
+// has always the same size.)
+static bool small_fits(dtb_block* b, int ctas)
+{
+    if (b->small_fit < 0) {
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = small_config(b, ctas, at);
+        int clusters = 0;
+        cudaError_t e = cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, k_small, &cfg);
+        if (e != cudaSuccess) cudaGetLastError();
+        b->small_fit = e == cudaSuccess && clusters > 0 ? 1 : 0;
+    }
+    return b->small_fit == 1;
+}
+
 // n steps of k_small and their statistics (rows row0.. of the outputs).  Device outputs are written
 // by the kernel itself; small host outputs go to pinned memory the same way, so that a call costs
 // one launch and one synchronisation.  nact_host: the propagated counts on the host (nullable).
@@ -1282,12 +1317,6 @@ constexpr int64_t kSmallHostValues = 8192;   // statistics values written to pin
 static int run_small(dtb_block* b, int ctas, int n, float noise_rate, int isolated, int64_t row0, float* sum_out,
                      float* mean_out, uint32_t* nact_out, int where, std::vector<uint32_t>* nact_host)
 {
-    static std::atomic<uint64_t> ready{0};                               // devices whose attribute is set
-    const uint64_t bit = 1ull << (b->device & 63);
-    if (!(ready.load() & bit)) {
-        CK(cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax));
-        ready.fetch_or(bit);
-    }
     const int nt = (int)((b->N + kWarpNeurons - 1) / kWarpNeurons);
     SmallArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -1302,17 +1331,8 @@ static int run_small(dtb_block* b, int ctas, int n, float noise_rate, int isolat
     a.nact0 = b->ds.sub_nact; a.nact1 = b->d_nact2;
     a.vsum0 = b->ds.sub_vsum; a.vsum1 = b->d_vsum2;
     a.unmapped0 = b->ds.unmapped_nact; a.unmapped1 = b->d_unmapped2;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(kSmallThreads);
-    cfg.dynamicSmemBytes = small_smem(a.tiles_per_cta, (int)a.cap);
-    cfg.stream = b->stream;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)ctas;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    const cudaLaunchConfig_t cfg = small_config(b, ctas, at);
     DevState s = b->ds;
     const size_t ns = (size_t)b->n_sub, nv = (size_t)n * ns;
     const bool pinned = (where == DTB_HOST && (int64_t)nv <= kSmallHostValues) || (where == DTB_DEVICE && nact_host);
@@ -1961,7 +1981,8 @@ int dtb_block_run(dtb_block* b, int n_steps, float noise_rate, int isolated, int
         const int m = choose_mode(b, mode);
         const int mm = resolve_method(b, m);
         const uint32_t cap = b->stats_cap;
-        const int small = small_ctas(b, mm, expected_activity(b, noise_rate, isolated));
+        int small = small_ctas(b, mm, expected_activity(b, noise_rate, isolated));
+        if (small > 0 && !small_fits(b, small)) small = 0;
         if (!small) RET(ensure_method(b, mm));
         int n;
         if (small > 0) {
