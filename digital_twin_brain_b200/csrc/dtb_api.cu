@@ -168,7 +168,7 @@ struct dtb_block {
     double pull_threshold = 0.05;
     int chunk = 32;
     int scatter_wpw = 0;          // bitmask words per warp in the push scatter (0: by network size)
-    int scatter_variant = -1;     // 1: targets prefetched into L2 before their reductions, 0: not, -1: by network size
+    int scatter_variant = 0;      // targets prefetched into L2 before their reductions: 0 by network size, 1 the other way
     int step_variant = 2;         // 0: 2 resident CTAs/SM register budget, 1: 3; 2..4: staged, 2..4 CTAs/SM
     // ordered push (bit-exact pull through per-neuron slots)
     bool has_qpos = false;
@@ -870,8 +870,7 @@ static int scatter_words(const dtb_block* b)
 // step 279 -> 267); while it does they only cost (1e6: 17.0 -> 21.3 us).
 static int scatter_form(const dtb_block* b)
 {
-    if (b->scatter_variant >= 0) return b->scatter_variant;
-    return 16 * b->N > ((int64_t)126 << 20) ? 1 : 0;
+    return (16 * b->N > ((int64_t)126 << 20) ? 1 : 0) ^ b->scatter_variant;
 }
 
 // how: kScatterJ (push), kScatterSlots / kScatterMasks (ordered push)
@@ -2193,7 +2192,7 @@ int dtb_block_get_tuning(dtb_block* b, int key, int64_t* value)
     case DTB_TUNE_STEP_VARIANT: *value = b->step_variant; break;
     case DTB_TUNE_PULL_METHOD: *value = b->pull_method; break;
     case DTB_TUNE_J_CACHE: *value = b->ds.j_keep; break;
-    case DTB_TUNE_SCATTER_VARIANT: *value = scatter_form(b); break;
+    case DTB_TUNE_SCATTER_VARIANT: *value = b->scatter_variant; break;
     case DTB_TUNE_PUSH_METHOD: *value = b->push_method; break;
     case DTB_TUNE_STAGE_WAIT_LIMIT: *value = b->ds.stage_wait_limit; break;
     case DTB_TUNE_SCATTER_REVERSE: *value = b->ds.rev_scatter; break;
@@ -2227,7 +2226,7 @@ int dtb_block_autotune(dtb_block* b, int n_steps, float noise_rate, float* repor
     }
     if (b->has_push) {
         const int cand[6] = {1, 2, 4, 8, 16, 32};
-        int best_sv = scatter_form(b);
+        int best_sv = b->scatter_variant;
         for (int sv = 0; sv < 2; ++sv)
             for (int w : cand) {
                 b->scatter_wpw = w;

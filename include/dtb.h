@@ -237,9 +237,9 @@ int dtb_block_time_kernels(dtb_block* b, int n_steps, float noise_rate, int isol
  *                          neurons propagate, else the streamed gather
  * DTB_TUNE_J_CACHE         0 = the update streams J (evict first), 1 = its J
  *                          stores keep normal L2 priority for the scatter
- * DTB_TUNE_SCATTER_VARIANT push scatter: 1 = the targets of a batch are prefetched into
- *                          L2 before their reductions, 0 = not (until set, 1 for networks
- *                          whose J exceeds L2)
+ * DTB_TUNE_SCATTER_VARIANT push scatter: 0 = the targets of a batch are prefetched into
+ *                          L2 before their reductions where J exceeds L2 and not where it
+ *                          fits (default), 1 = the other way round
  * DTB_TUNE_PUSH_METHOD     how DTB_MODE_PUSH adds the weights of firing rows
  *                          (the order of the float additions differs, the sums
  *                          agree to rounding): 1 = one float2 atomic into J per

@@ -41,3 +41,16 @@ def test_push_scatter_shapes(words, variant, reverse):
     assert a.get(FIELD_EVENTS) == b.get(FIELD_EVENTS)
     # 40 steps of up to ~25 additions in another order: 1000 float32 roundings at most
     np.testing.assert_allclose(a.get(FIELD_J), b.get(FIELD_J), rtol=1e-5, atol=1e-5)
+
+
+def test_scatter_variant_zero_is_the_default():
+    """Also for a network whose J exceeds L2 (16 bytes a neuron): setting the default changes nothing."""
+    net = Network.from_spec(synthetic.single_block(8_400_000, 2, gen_seed=4), device=0)
+    assert net.get_tuning(TUNE_SCATTER_VARIANT) == 0
+    took = []
+    for _ in range(2):
+        net.run(8, noise_rate=0.02, isolated=True, mode="push", out=None)
+        took.append(net.info().kernel_launches)
+        net.set_tuning(TUNE_SCATTER_VARIANT, 0)
+        assert net.get_tuning(TUNE_SCATTER_VARIANT) == 0
+    assert took[1] == 2 * took[0]
