@@ -120,6 +120,9 @@ void default_decay(const float* prop, float dt, float* out)
 }  // namespace
 
 // ------------------------------------------------------------ handle
+constexpr int kStepVariant = 2;
+constexpr uint32_t kStageWaitLimit = 1u << 20;
+
 struct dtb_block {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -169,7 +172,7 @@ struct dtb_block {
     int chunk = 32;
     int scatter_wpw = 0;          // bitmask words per warp in the push scatter (0: by network size)
     int scatter_variant = 0;      // targets prefetched into L2 before their reductions: 0 by network size, 1 the other way
-    int step_variant = 2;         // 0: 2 resident CTAs/SM register budget, 1: 3; 2..4: staged, 2..4 CTAs/SM
+    int step_variant = kStepVariant;   // 0: 2 resident CTAs/SM register budget, 1: 3; 2..4: staged, 2..4 CTAs/SM
     // ordered push (bit-exact pull through per-neuron slots)
     bool has_qpos = false;
     int pull_method = 0;          // 0: auto, 1: row gather, 2: ordered push (slots), 3: (masks), 4: streamed gather
@@ -197,7 +200,7 @@ struct dtb_block {
     uint32_t* d_unmapped2 = nullptr;
     int small_fit = -1;           // the device can place its cluster (-1: not asked yet)
     int grp_n_sub = -1;           // subblocks when the statistics groups were built
-    bool knobs_set = false;       // the caller chose a schedule (dtb_block_set_tuning): launch per step as asked
+    uint32_t knobs = 0;           // keys the caller set to other than their defaults: bit per DTB_TUNE_*
     bool chunk_set = false;
     // attached BOLD
     int bold_R = 0;
@@ -389,7 +392,7 @@ static int alloc_state(dtb_block* b)
     s.seed = b->seed;
     s.stream_id = b->stream_id;
     s.dt = b->dt;
-    s.stage_wait_limit = 1u << 20;
+    s.stage_wait_limit = kStageWaitLimit;
     s.forced_active = nullptr;
     s.forced_new = nullptr;
     return DTB_OK;
@@ -858,12 +861,16 @@ static int launch_gather_only(dtb_block* b, const DevState& s, int gather = kGat
 // should not queue behind each other) and at most four words, past which a warp's rows serialise.
 // Measured, N = 31,013: 1 / 4 / 32 words 9.0 / 10.8 / 16.3 us; 1e6: 25.2 / 19.9 / 27.2; 1.2e7:
 // 226 / 196 / 243 (the row-list kernel).
-static int scatter_words(const dtb_block* b)
+static int words_by_size(const dtb_block* b)
 {
-    if (b->scatter_wpw > 0) return b->scatter_wpw;
     int w = 1;
     while (w < 4 && b->ds.n_words >= (int64_t)8192 * w) w *= 2;
     return w;
+}
+
+static int scatter_words(const dtb_block* b)
+{
+    return b->scatter_wpw > 0 ? b->scatter_wpw : words_by_size(b);
 }
 
 // Prefetched targets pay once J no longer fits L2 (1.2e7 neurons, 195 MB of J: scatter 195 -> 180 us,
@@ -1222,6 +1229,12 @@ static int emit_stats(dtb_block* b, int rows, int64_t row0, float* sum_out, floa
     return DTB_OK;
 }
 
+// Keys that choose how the per-step kernels run: set to other than their defaults, these kernels run.
+constexpr uint32_t knob(int key) { return 1u << key; }
+constexpr uint32_t kStepKnobs = knob(DTB_TUNE_SCATTER_WORDS) | knob(DTB_TUNE_STEP_VARIANT) | knob(DTB_TUNE_J_CACHE) |
+                                knob(DTB_TUNE_SCATTER_VARIANT) | knob(DTB_TUNE_SCATTER_REVERSE) |
+                                knob(DTB_TUNE_STAGE_WAIT_LIMIT);
+
 // The fraction of neurons that a run's steps are expected to propagate: the noise of the call plus
 // what earlier runs showed beyond theirs (spikes); before any did, 1 % of the neurons.
 static double noise_of(const dtb_block* b, float noise_rate)
@@ -1263,7 +1276,8 @@ static int small_ctas(const dtb_block* b, int method, double f)
     if (b->N <= 0 || b->N > kSmallMaxNeurons) return 0;
     if (method != DTB_MODE_PUSH && method != kModeSlots) return 0;
     if (method == kModeSlots && b->pull_method != 0) return 0;           // the caller asked for the slot kernels
-    if (b->knobs_set || !b->use_graphs) return 0;
+    if (!b->use_graphs || (b->knobs & kStepKnobs)) return 0;             // a schedule of the step kernels
+    if (method == DTB_MODE_PUSH && (b->knobs & knob(DTB_TUNE_PUSH_METHOD))) return 0;
     if (!b->has_pull || !b->has_push || !b->has_qpos) return 0;
     if (b->override_live || s.gnrn || s.n_src > 0 || s.forced_active) return 0;   // the general update
     if (!staged_layout(s) || !s.tile_cls || b->grp_n_sub != b->n_sub) return 0;
@@ -2173,10 +2187,17 @@ int dtb_block_set_tuning(dtb_block* b, int key, int64_t value)
     }
     default: return fail(DTB_ERR_ARG, "unknown tuning key %d", key);
     }
-    if (key == DTB_TUNE_CHUNK) b->chunk_set = true;
-    else if (key != DTB_TUNE_PULL_THRESHOLD_PPM && key != DTB_TUNE_PULL_METHOD && key != DTB_TUNE_PUSH_METHOD &&
-             key != DTB_TUNE_USE_GRAPHS)
-        b->knobs_set = true;
+    bool own = true;   // other than the default
+    switch (key) {
+    case DTB_TUNE_CHUNK: b->chunk_set = true; break;
+    case DTB_TUNE_SCATTER_WORDS: own = value != words_by_size(b); break;
+    case DTB_TUNE_STEP_VARIANT: own = value != kStepVariant; break;
+    case DTB_TUNE_STAGE_WAIT_LIMIT: own = value != (int64_t)kStageWaitLimit; break;
+    case DTB_TUNE_J_CACHE:
+    case DTB_TUNE_SCATTER_VARIANT:
+    case DTB_TUNE_SCATTER_REVERSE: own = value != 0; break;
+    }
+    b->knobs = own ? b->knobs | knob(key) : b->knobs & ~knob(key);
     drop_graphs(b);
     return DTB_OK;
 }

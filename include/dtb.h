@@ -207,10 +207,16 @@ int dtb_block_step_forced(dtb_block* b, float noise_rate, int isolated, int mode
 int dtb_block_time_kernels(dtb_block* b, int n_steps, float noise_rate, int isolated, int mode, float* out_ms);
 
 /* Schedule knobs (new: the reference has a fixed launch shape per kernel).
+ * Networks of up to 12,288 neurons run their steps in one cluster launch while the few SMs of a cluster
+ * are the better place for their synaptic events (expected from the call's noise and the activity of
+ * earlier runs); the results are the same, and push then adds in pull order.  Their steps run through
+ * the per-step kernels while a key that shapes these (SCATTER_WORDS, STEP_VARIANT, J_CACHE,
+ * SCATTER_VARIANT, SCATTER_REVERSE, STAGE_WAIT_LIMIT) is set to other than its default, with USE_GRAPHS
+ * 0, in pull mode with a PULL_METHOD other than 0, and in push mode once PUSH_METHOD was set.
+ * dtb_block_time_kernels and dtb_block_autotune always time the per-step kernels; what autotune adopts
+ * is the schedule that these run with and does not keep a network from the cluster launch.
  * DTB_TUNE_SCATTER_WORDS   bitmask words per warp in the push scatter (1..32; until
  *                          set, 1, 2 or 4 by the network's size)
- * Networks of up to 12,288 neurons run their steps in one cluster launch unless one of
- * the schedule keys below was set (the results are the same).
  * DTB_TUNE_CHUNK           steps per captured CUDA graph (1..4096)
  * DTB_TUNE_PULL_THRESHOLD_PPM  activity fraction (parts per million of the
  *                          neurons propagating per step) above which

@@ -6,7 +6,9 @@ import pytest
 
 from digital_twin_brain_b200 import Network, synthetic
 from digital_twin_brain_b200._lib import (FIELD_ACTIVE, FIELD_EVENTS, FIELD_I_SYN, FIELD_J, FIELD_NEW_ACTIVE, FIELD_T,
-                                          FIELD_T_LAST, FIELD_V, TUNE_PULL_METHOD)
+                                          FIELD_T_LAST, FIELD_V, TUNE_BIN_WORDS, TUNE_J_CACHE, TUNE_PULL_METHOD,
+                                          TUNE_PUSH_METHOD, TUNE_SCATTER_REVERSE, TUNE_SCATTER_VARIANT,
+                                          TUNE_SCATTER_WORDS, TUNE_STAGE_WAIT_LIMIT, TUNE_STEP_VARIANT, TUNE_USE_GRAPHS)
 
 pytestmark = pytest.mark.gpu
 ROWS = 1
@@ -101,3 +103,31 @@ def test_loop_follows_the_activity_seen():
     driven, f = launches(40)
     assert f > 0.04 and first < 2 * 300
     assert quiet == 1 and driven >= 80
+
+
+def test_schedule_keys_choose_the_kernels():
+    """A key of the per-step kernels set to its default, or back to it, keeps the loop; another value,
+    or an explicit push method, selects these kernels."""
+    net = Network.from_spec(synthetic.single_block(3000, 40, gen_seed=3), device=0)
+
+    def loop(mode="push"):
+        before = net.info().kernel_launches
+        net.run(10, noise_rate=0.01, mode=mode)
+        return net.info().kernel_launches - before == 1
+    others = {TUNE_SCATTER_WORDS: 8, TUNE_STEP_VARIANT: 0, TUNE_J_CACHE: 1, TUNE_SCATTER_VARIANT: 1,
+              TUNE_SCATTER_REVERSE: 1, TUNE_STAGE_WAIT_LIMIT: 5, TUNE_USE_GRAPHS: 0}
+    for key, other in others.items():
+        default = net.get_tuning(key)
+        net.set_tuning(key, default)
+        assert loop("push") and loop("pull"), key
+        net.set_tuning(key, other)
+        assert not loop("push") and not loop("pull"), key
+        net.set_tuning(key, default)
+        assert loop("push"), key
+    assert net.get_tuning(TUNE_SCATTER_VARIANT) == 0
+    net.set_tuning(TUNE_BIN_WORDS, 64)           # a key of the binned push alone
+    assert loop("push")
+    net.autotune(4, noise_rate=0.01)
+    assert loop("push") and loop("pull")
+    net.set_tuning(TUNE_PUSH_METHOD, 1)          # atomics into J, asked for
+    assert not loop("push") and loop("pull")
