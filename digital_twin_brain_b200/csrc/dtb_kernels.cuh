@@ -116,12 +116,12 @@ __device__ __forceinline__ void add_events(const DevState& s, unsigned long long
     else atomicAdd(&s.ctl->events, ev);
 }
 
-// (A plain load: the bitmask was written by a kernel this one may overlap the start of, so not the
-// read-only path.)
+// NC: through the read-only path, for kernels that start after the one that wrote the bitmask has
+// ended; a kernel that may have been launched before (launch_chain) takes a plain load.
+template <bool NC>
 __device__ __forceinline__ bool test_bit(const uint32_t* bits, int64_t n)
 {
-    uint32_t w;
-    asm volatile("ld.global.u32 %0, [%1];" : "=r"(w) : "l"(bits + (n >> 5)));
+    const uint32_t w = NC ? __ldg(bits + (n >> 5)) : bits[n >> 5];
     return (w >> (n & 31)) & 1u;
 }
 
@@ -129,6 +129,7 @@ __device__ __forceinline__ bool test_bit(const uint32_t* bits, int64_t n)
 // Sum of the weights of row n whose presynaptic neuron is set in `bits`,
 // accumulated strictly in row order from +0 (sparse.mm order). All lanes
 // return the same value.
+template <bool NC>
 __device__ __forceinline__ float4 gather_row(const DevState& s, const uint32_t* bits, int64_t n,
                                              int lane, uint32_t& events)
 {
@@ -139,7 +140,7 @@ __device__ __forceinline__ float4 gather_row(const DevState& s, const uint32_t* 
         const int64_t idx = e + lane;
         const bool valid = idx < e1;
         const uint32_t c = valid ? __ldg(s.pcol + idx) : 0u;
-        const bool act = valid && test_bit(bits, c & kIndexMask);
+        const bool act = valid && test_bit<NC>(bits, c & kIndexMask);
         unsigned m = __ballot_sync(0xffffffffu, act);
         events += __popc(m);
         float2 w = make_float2(0.0f, 0.0f);
@@ -1018,7 +1019,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
                         const int l = __ffs(m) - 1;
                         m &= m - 1;
                         uint32_t ev = 0;
-                        const float4 a = gather_row(s, gbits, base + j * 32 + l, lane, ev);
+                        const float4 a = gather_row<false>(s, gbits, base + j * 32 + l, lane, ev);
                         if (lane == l) sum = a;
                     }
                     Jn[j] = add4(Jn[j], sum);   // models/block.py:71-73
@@ -1057,7 +1058,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
 #pragma unroll
                 for (int u = 0; u < UC; ++u) {
                     const int64_t e = c + u * 32 + lane;
-                    act[u] = e < e1 && test_bit(gbits, col[u] & kIndexMask);
+                    act[u] = e < e1 && test_bit<true>(gbits, col[u] & kIndexMask);
                 }
 #pragma unroll
                 for (int u = 0; u < UC; ++u) {
@@ -1132,7 +1133,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
                 for (int r = 0; r < 32; ++r) {
                     const int64_t n = base + j * 32 + r;
                     if (n >= s.N) break;
-                    const float4 a = gather_row(s, gbits, n, lane, events);
+                    const float4 a = gather_row<true>(s, gbits, n, lane, events);
                     if (lane == r) sum[j] = a;
                 }
             }
@@ -1156,11 +1157,12 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
         const uint32_t tcls = s.tile_cls ? __ldg(s.tile_cls + tile) : kMixedTile;   // the tile's class, or kMixedTile
         const bool mixed = tcls == kMixedTile;
         bool lean = false;
-        if (!FORCED && !mixed && base + kWarpNeurons <= s.N && s.j_es == 1 && (!STAGED || staged)) {
+        if (!FORCED && GATHER != kGatherStream && !mixed && base + kWarpNeurons <= s.N && s.j_es == 1 && (!STAGED || staged)) {
             // A whole tile of one class, the plain form: the ALU pipe (compares, selects, bit operations)
             // bounds the update, so no per-neuron guards, the firing masks are ballots of the predicates
             // themselves, the minimum with V_th is the threshold test's select, and the noise test an
-            // integer compare.
+            // integer compare.  (Not after the streamed gather, which has 20 times the update's work and
+            // whose loop compiles 4 % slower beside this form: 1e6 neurons, p = 0.2: 2114 -> 2196 us.)
             const ParamClass p = load_class(s.pc, tcls);
             if (p.sub >= 0 && p.sub < s.n_sub && !isnan(p.Vth)) {
                 lean = true;
