@@ -172,7 +172,7 @@ struct dtb_block {
     int chunk = 32;
     int scatter_wpw = 0;          // bitmask words per warp in the push scatter (0: by network size)
     int scatter_variant = 0;      // targets prefetched into L2 before their reductions: 0 by network size, 1 the other way
-    int step_variant = kStepVariant;   // 0: 2 resident CTAs/SM register budget, 1: 3; 2..4: staged, 2..4 CTAs/SM
+    int step_variant = -1;        // 0: 2 resident CTAs/SM register budget, 1: 3; 2..4: staged, 2..4 CTAs/SM; -1: variant_of
     // ordered push (bit-exact pull through per-neuron slots)
     bool has_qpos = false;
     int pull_method = 0;          // 0: auto, 1: row gather, 2: ordered push (slots), 3: (masks), 4: streamed gather
@@ -764,28 +764,37 @@ static void launch_step_bins_staged(dtb_block* b, const DevState& s)
 
 static bool staged_layout(const DevState& s);
 
+// The update's variant, until one is chosen: staged with two CTAs per SM (1.2e7 neurons, a push step:
+// 279 -> 267 us against three), with three where it folds the bins of a binned push first (6e6 neurons
+// 228 -> 217 us a step, 1.28e6 in 64 members 75.7 -> 72.7, 1e6 in one region 77.2 -> 77.7).
+static int variant_of(const dtb_block* b, bool bins)
+{
+    return b->step_variant >= 0 ? b->step_variant : (bins ? 3 : kStepVariant);
+}
+
 template <int G, bool U, bool F>
 static void launch_step(dtb_block* b, const DevState& s)
 {
+    const int v = variant_of(b, G == kGatherBins);
     if constexpr (G == kGatherBins) {
         if constexpr (U) {
             // step variants 2..4 stage the state (bins of 1024 neurons, split J planes)
-            if (b->step_variant >= 2 && s.bin_shift == kBinMinShift && staged_layout(s)) {
-                if (b->step_variant == 2) launch_step_bins_staged<F, 2>(b, s);
+            if (v >= 2 && s.bin_shift == kBinMinShift && staged_layout(s)) {
+                if (v == 2) launch_step_bins_staged<F, 2>(b, s);
                 else launch_step_bins_staged<F, 3>(b, s);
                 return;
             }
         }
-        if (b->step_variant == 1 || b->step_variant >= 3) launch_step_bins<U, F, 3>(b, s);
+        if (v == 1 || v >= 3) launch_step_bins<U, F, 3>(b, s);
         else launch_step_bins<U, F, 2>(b, s);
         return;
     }
     if constexpr (G == 0) {
-        if (b->step_variant == 2 && staged_layout(s)) { launch_step_staged<U, F, 2>(b, s); return; }
-        if (b->step_variant == 3 && staged_layout(s)) { launch_step_staged<U, F, 3>(b, s); return; }
-        if (b->step_variant == 4 && staged_layout(s)) { launch_step_staged<U, F, 4>(b, s); return; }
+        if (v == 2 && staged_layout(s)) { launch_step_staged<U, F, 2>(b, s); return; }
+        if (v == 3 && staged_layout(s)) { launch_step_staged<U, F, 3>(b, s); return; }
+        if (v == 4 && staged_layout(s)) { launch_step_staged<U, F, 4>(b, s); return; }
     }
-    if (b->step_variant == 1) launch_step_m<G, U, F, 3>(b, s);
+    if (v == 1) launch_step_m<G, U, F, 3>(b, s);
     else launch_step_m<G, U, F, 2>(b, s);
 }
 
@@ -2214,7 +2223,7 @@ int dtb_block_get_tuning(dtb_block* b, int key, int64_t* value)
     case DTB_TUNE_CHUNK: *value = b->chunk; break;
     case DTB_TUNE_PULL_THRESHOLD_PPM: *value = (int64_t)std::llround(b->pull_threshold * 1e6); break;
     case DTB_TUNE_USE_GRAPHS: *value = b->use_graphs ? 1 : 0; break;
-    case DTB_TUNE_STEP_VARIANT: *value = b->step_variant; break;
+    case DTB_TUNE_STEP_VARIANT: *value = variant_of(b, use_bins(b)); break;
     case DTB_TUNE_PULL_METHOD: *value = b->pull_method; break;
     case DTB_TUNE_J_CACHE: *value = b->ds.j_keep; break;
     case DTB_TUNE_SCATTER_VARIANT: *value = b->scatter_variant; break;

@@ -183,3 +183,14 @@ def test_binned_staged_copy_given_up():
     a.set_tuning(TUNE_STAGE_WAIT_LIMIT, 1 << 20)
     a.run(5, mode="push")
     a.synchronize()
+
+
+def test_update_variant_follows_the_push_method():
+    net = Network.from_spec(synthetic.single_block(20000, 30, name="n20k_v"), device=0)
+    assert net.get_tuning(TUNE_STEP_VARIANT) == 2
+    net.set_tuning(TUNE_PUSH_METHOD, BINNED)
+    assert net.get_tuning(TUNE_STEP_VARIANT) == 3
+    net.set_tuning(TUNE_STEP_VARIANT, 0)
+    assert net.get_tuning(TUNE_STEP_VARIANT) == 0
+    net.set_tuning(TUNE_PUSH_METHOD, ATOMIC)
+    assert net.get_tuning(TUNE_STEP_VARIANT) == 0
