@@ -161,6 +161,9 @@ struct dtb_block {
     // pinned host staging
     void* pinned = nullptr;
     size_t pinned_bytes = 0;
+    // the run parameters queued last (set_run_params)
+    bool run_set = false, run_isolated = false, run_replayed = false;
+    float run_rate = 0.0f;
     // auto mode
     int64_t launches = 0;
     uint64_t samples_from = 0;    // step at which sampling started
@@ -821,11 +824,13 @@ static int launch_src(dtb_block* b, const DevState& s)
 
 // gather: 0 none, kGatherRows (fused pull gather), kGatherSlots / kGatherMasks (ordered push)
 // defer: a scatter launched with the same flag follows and folds the step's statistics.
-static int launch_update(dtb_block* b, const DevState& s_in, int gather, bool forced, bool defer = false)
+// last: the step ends its run (the next one's statistics start at row 0).
+static int launch_update(dtb_block* b, const DevState& s_in, int gather, bool forced, bool last, bool defer = false)
 {
     if (s_in.N <= 0) return DTB_OK;
     DevState s = s_in;
     s.defer = defer ? 1 : 0;
+    s.last = last ? 1 : 0;
     if (s.n_src > 0 && s.forced_active == s.src_val) {   // input neurons replay their raster
         RET(launch_src(b, s));
         forced = true;
@@ -894,8 +899,10 @@ static int scatter_form(const dtb_block* b)
 }
 
 // how: kScatterJ (push), kScatterSlots / kScatterMasks (ordered push)
-static int launch_scatter(dtb_block* b, const DevState& s, int how = kScatterJ, bool defer = false)
+static int launch_scatter(dtb_block* b, const DevState& s_in, int how = kScatterJ, bool defer = false, bool last = false)
 {
+    DevState s = s_in;
+    s.last = last ? 1 : 0;
     const int wpw = scatter_words(b);
     const int64_t warps = (s.n_words + wpw - 1) / wpw;
     const int stat = defer ? std::max(1, (int)grid_for(s.n_groups, kStatThreads)) : 0;
@@ -1070,26 +1077,25 @@ static int enqueue_steps(dtb_block* b, int n, int mode)
     const bool defer = can_defer(b);
     if (mode == DTB_MODE_PUSH) {
         for (int k = 0; k < n; ++k) {
-            RET(launch_update(b, s, 0, false, defer));
-            RET(launch_scatter(b, s, kScatterJ, defer));
+            RET(launch_update(b, s, 0, false, k + 1 == n, defer));
+            RET(launch_scatter(b, s, kScatterJ, defer, k + 1 == n));
         }
     } else if (mode == kModeBinned) {
         for (int k = 0; k < n; ++k) {
-            RET(launch_update(b, s, kGatherBins, false));
+            RET(launch_update(b, s, kGatherBins, false, k + 1 == n));
             RET(launch_bin_scatter(b, s));
         }
     } else if (mode == kModeSlots || mode == kModeMasks) {
         const int g = mode == kModeSlots ? kGatherSlots : kGatherMasks;
         const int how = mode == kModeSlots ? kScatterSlots : kScatterMasks;
         for (int k = 0; k < n; ++k) {
-            RET(launch_update(b, s, k ? g : 0, false, defer));
-            RET(launch_scatter(b, s, how, defer));
+            RET(launch_update(b, s, k ? g : 0, false, k + 1 == n, defer));
+            RET(launch_scatter(b, s, how, defer, k + 1 == n));
         }
         RET(launch_gather_only(b, s, g));
     } else {
         const int g = mode == kModeStream ? kGatherStream : kGatherRows;
-        RET(launch_update(b, s, 0, false));
-        for (int k = 1; k < n; ++k) RET(launch_update(b, s, g, false));
+        for (int k = 0; k < n; ++k) RET(launch_update(b, s, k ? g : 0, false, k + 1 == n));
         RET(launch_gather_only(b, s, g));
     }
     return DTB_OK;
@@ -1183,10 +1189,30 @@ static int ensure_method(dtb_block* b, int mm)
     return DTB_OK;
 }
 
+// The device's clock as the host sets it: the next step is the first of a run.
+static int upload_steps(dtb_block* b)
+{
+    static_assert(offsetof(Ctl, steps_done) == 0 && offsetof(Ctl, run_base) == 8, "Ctl layout");
+    const uint64_t v[2] = {b->steps, b->steps};
+    CK(cudaMemcpyAsync(b->ds.ctl, v, sizeof(v), cudaMemcpyHostToDevice, b->stream));
+    CK(cudaStreamSynchronize(b->stream));
+    return DTB_OK;
+}
+
+// The noise rate and isolation of the steps queued behind it, where they differ from the last ones
+// queued.  In a CUDA graph of the caller's they always go along, and from then on everywhere: a replay
+// may have come in between.
 static int set_run_params(dtb_block* b, float noise_rate, int isolated)
 {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (!b->run_replayed && (cudaStreamIsCapturing(b->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone))
+        b->run_replayed = true;
+    if (!b->run_replayed && b->run_set && b->run_rate == noise_rate && b->run_isolated == (isolated != 0)) return DTB_OK;
     k_set_run<<<1, 1, 0, b->stream>>>(b->ds.ctl, noise_rate, isolated ? 1 : 0);
     CK(cudaGetLastError());
+    b->run_set = true;
+    b->run_rate = noise_rate;
+    b->run_isolated = isolated != 0;
     return DTB_OK;
 }
 
@@ -2072,7 +2098,7 @@ int dtb_block_time_kernels(dtb_block* b, int n_steps, float noise_rate, int isol
     }
     if (m == kModeBinned) {
         for (int st = 0; st < n_steps && rc == DTB_OK && k + 6 <= n_ev; ++st) {
-            rec(k); rc = launch_update(b, b->ds, kGatherBins, false); rec(k + 1);
+            rec(k); rc = launch_update(b, b->ds, kGatherBins, false, st + 1 == n_steps); rec(k + 1);
             kind.push_back(0); k += 2;
             if (rc != DTB_OK) break;
             rec(k); rc = launch_bin_scatter(b, b->ds); rec(k + 1); kind.push_back(1); k += 2;
@@ -2084,10 +2110,10 @@ int dtb_block_time_kernels(dtb_block* b, int n_steps, float noise_rate, int isol
         const int g = m == kModeSlots ? kGatherSlots : kGatherMasks;
         const int how = m == kModeSlots ? kScatterSlots : (m == kModeMasks ? kScatterMasks : kScatterJ);
         for (int st = 0; st < n_steps && rc == DTB_OK && k + 6 <= n_ev; ++st) {
-            rec(k); rc = launch_update(b, b->ds, (ord && st > 0) ? g : 0, false, can_defer(b)); rec(k + 1);
+            rec(k); rc = launch_update(b, b->ds, (ord && st > 0) ? g : 0, false, st + 1 == n_steps, can_defer(b)); rec(k + 1);
             kind.push_back(0); k += 2;
             if (rc != DTB_OK) break;
-            rec(k); rc = launch_scatter(b, b->ds, how, can_defer(b)); rec(k + 1); kind.push_back(1); k += 2;
+            rec(k); rc = launch_scatter(b, b->ds, how, can_defer(b), st + 1 == n_steps); rec(k + 1); kind.push_back(1); k += 2;
             done_steps++;
         }
         if (ord && rc == DTB_OK) {
@@ -2095,9 +2121,9 @@ int dtb_block_time_kernels(dtb_block* b, int n_steps, float noise_rate, int isol
         }
     } else {
         const int g = m == kModeStream ? kGatherStream : kGatherRows;
-        rec(k); rc = launch_update(b, b->ds, 0, false); rec(k + 1); kind.push_back(0); k += 2;
+        rec(k); rc = launch_update(b, b->ds, 0, false, n_steps == 1); rec(k + 1); kind.push_back(0); k += 2;
         for (int st = 1; st < n_steps && rc == DTB_OK && k + 4 <= n_ev; ++st) {
-            rec(k); rc = launch_update(b, b->ds, g, false); rec(k + 1); kind.push_back(0); k += 2;
+            rec(k); rc = launch_update(b, b->ds, g, false, st + 1 == n_steps); rec(k + 1); kind.push_back(0); k += 2;
         }
         if (rc == DTB_OK) { rec(k); rc = launch_gather_only(b, b->ds, g); rec(k + 1); kind.push_back(1); k += 2; }
         done_steps = (int)kind.size() - 1;
@@ -2360,12 +2386,12 @@ int dtb_block_step_forced(dtb_block* b, float noise_rate, int isolated, int mode
     if (mm == kModeBinned) {
         s.bin_idx = b->ds.bin_idx; s.bin_w = b->ds.bin_w; s.bin_cnt = b->ds.bin_cnt;
         s.n_bins = b->ds.n_bins; s.bin_cap = b->ds.bin_cap; s.bin_shift = b->ds.bin_shift;
-        RET(launch_update(b, s, kGatherBins, true));
+        RET(launch_update(b, s, kGatherBins, true, true));
         RET(launch_bin_scatter(b, s));
         b->bins_pending = true;
     } else {
         RET(flush_bins(b));
-        RET(launch_update(b, s, 0, true));
+        RET(launch_update(b, s, 0, true, true));
         if (m == DTB_MODE_PUSH) RET(launch_scatter(b, s));
         else RET(launch_gather_only(b, s));
     }
@@ -2499,7 +2525,7 @@ int dtb_block_set(dtb_block* b, int field, const void* src, int where)
         if (where == DTB_HOST) std::memcpy(&v, src, 8);
         else CK(cudaMemcpy(&v, src, 8, cudaMemcpyDeviceToHost));
         b->steps = v;
-        CK(cudaMemcpyAsync(&s.ctl->steps_done, &b->steps, sizeof(uint64_t), cudaMemcpyHostToDevice, b->stream));
+        RET(upload_steps(b));
         break;
     }
     default: return fail(DTB_ERR_ARG, "field %d cannot be set", field);
@@ -2816,10 +2842,10 @@ int dtb_block_load(dtb_block* b, const char* path)
     CK(cudaMemcpy(b->ds.J2 + b->ds.j_ps, reinterpret_cast<const float2*>(J.data()) + N, 8 * N, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(b->ds.tlast, T.data(), 4 * N, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(&b->ds.ctl->t, &t, 4, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(&b->ds.ctl->steps_done, &steps, 8, cudaMemcpyHostToDevice));
+    b->steps = steps;
+    RET(upload_steps(b));
     CK(cudaMemcpy(&b->ds.ctl->use_isyn_override, &ov, 4, cudaMemcpyHostToDevice));
     if (ov) CK(cudaMemcpy(b->ds.isyn_override, I.data(), 4 * N, cudaMemcpyHostToDevice));
-    b->steps = steps;
     b->override_pending = false;
     b->override_live = ov != 0;
     return DTB_OK;

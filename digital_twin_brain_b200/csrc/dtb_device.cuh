@@ -60,8 +60,8 @@ static_assert(sizeof(ParamClass) == 96, "ParamClass layout");
 // last CTA of each update kernel.
 struct Ctl {
     unsigned long long steps_done;   // number of completed updates (Philox step counter)
-    // per-run parameters (k_set_run)
-    unsigned long long run_base;     // steps_done at the start of the current run (stats row 0)
+    unsigned long long run_base;     // steps_done at the start of the current run (stats row 0; DevState::last)
+    // run parameters (k_set_run)
     float noise_rate;                // >= 0: scalar rate; < 0: per-class rate
     int32_t isolated;                // block.run(isolated=...)
     float t;                         // block.t after the last update (float32 accumulation)
@@ -69,7 +69,7 @@ struct Ctl {
     uint32_t stats_cap;              // rows of the per-step stats buffers
     uint32_t use_isyn_override;      // next update takes I_syn from isyn_override
     uint32_t err;                    // sticky error flags
-    uint32_t pad;
+    uint32_t row;                    // statistics row of the step just taken, for the kernel that follows
     unsigned long long events;       // synaptic events propagated since creation
     unsigned long long step_cur;     // deferred statistics: the step of the latest update, whose clock the
                                      // scatter that follows advances
@@ -149,6 +149,7 @@ struct DevState {
     uint32_t* unmapped_nact;    // new_active of neurons whose subblock is out of range
     unsigned long long* win_spk; // [n_sub] spikes accumulated since the host last cleared them
     int stats_ext;              // 1: statistics and BOLD in k_stats (many subblocks / regions)
+    int last;                   // 1: the step ends its run: the next one's statistics start at row 0
     int defer;                  // 1: a scatter follows this update; its first CTAs fold the statistics,
                                 // run BOLD and advance the clock
     const int32_t* grp_ptr;     // k_stats groups: [n_groups+1] into grp_sub

@@ -335,6 +335,9 @@ __device__ __forceinline__ void bold_region_step(const BoldDev& b, int r, double
 // Runs in the last CTA of an update kernel: per-subblock statistics of step
 // `steps_done` (models/block.py:144-150), BOLD (simulation/simulation.py:
 // 269-279 + models/bold_model_pytorch.py:43-78 in float64), clock advance.
+// A statistics row as Ctl::row holds it (rows past the buffers are not written).
+__device__ __forceinline__ uint32_t stats_row(unsigned long long row) { return row < 0xffffffffull ? (uint32_t)row : 0xffffffffu; }
+
 __device__ void step_epilogue(const DevState& s, unsigned long long steps_done, float t)
 {
     Ctl* ctl = s.ctl;
@@ -347,6 +350,8 @@ __device__ void step_epilogue(const DevState& s, unsigned long long steps_done, 
             ctl->use_isyn_override = 0u;
             ctl->done = 0u;
             ctl->steps_done = steps_done + 1ull;
+            ctl->row = stats_row(row);
+            if (s.last) ctl->run_base = steps_done + 1ull;
             __threadfence();
         }
         return;
@@ -389,6 +394,7 @@ __device__ void step_epilogue(const DevState& s, unsigned long long steps_done, 
         ctl->use_isyn_override = 0u;
         ctl->done = 0u;
         ctl->steps_done = steps_done + 1ull;
+        if (s.last) ctl->run_base = steps_done + 1ull;
         __threadfence();
     }
 }
@@ -433,7 +439,7 @@ __device__ __forceinline__ void stats_group(const DevState& s, int g, unsigned l
 
 __global__ void __launch_bounds__(kStatThreads) k_stats(DevState s)
 {
-    const unsigned long long row = s.ctl->steps_done - 1ull - s.ctl->run_base;   // clock already advanced
+    const unsigned long long row = s.ctl->row;
     stats_group(s, blockIdx.x * blockDim.x + threadIdx.x, row, row < (unsigned long long)s.ctl->stats_cap);
 }
 
@@ -444,7 +450,7 @@ __device__ __forceinline__ void deferred_stats(const DevState& s)
 {
     Ctl* ctl = s.ctl;
     const unsigned long long step = ctl->step_cur;
-    const unsigned long long row = step - ctl->run_base;
+    const unsigned long long row = ctl->row;
     const bool write = row < (unsigned long long)ctl->stats_cap;
     stats_group(s, blockIdx.x * blockDim.x + threadIdx.x, row, write);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -453,16 +459,15 @@ __device__ __forceinline__ void deferred_stats(const DevState& s)
         ctl->t = __fadd_rn(ctl->t, s.dt);
         ctl->use_isyn_override = 0u;
         ctl->steps_done = step + 1ull;
+        if (s.last) ctl->run_base = step + 1ull;
     }
 }
 
 // The parameters of the steps queued behind it: arguments by value, so that the calls and chunks
 // queued before these steps, and a replay of a caller's graph, each keep their own (a copy from one
-// host buffer would be read when the stream gets there).  Launched outside the step chain: the clock
-// it reads is the last step's.
+// host buffer would be read when the stream gets there).
 __global__ void k_set_run(Ctl* ctl, float noise_rate, int32_t isolated)
 {
-    ctl->run_base = ctl->steps_done;
     ctl->noise_rate = noise_rate;
     ctl->isolated = isolated;
 }
@@ -677,6 +682,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
     if (UPDATE && s.defer && blockIdx.x == 0 && threadIdx.x == 0) {
         const unsigned long long row = steps_done - ctl->run_base;
         s.ctl->step_cur = steps_done;
+        s.ctl->row = stats_row(row);
         if (row < (unsigned long long)ctl->stats_cap) s.st_nact[row] = 0u;
     }
     const float t = UPDATE ? __fadd_rn(ctl->t, s.dt) : 0.0f;

@@ -519,6 +519,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(DevState s, SmallArg
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             s.ctl->t = t;
             s.ctl->steps_done = step0 + (unsigned long long)k;
+            s.ctl->run_base = step0 + (unsigned long long)k;
         }
         // the last step's slots into J, which a run leaves complete; the state back to global memory
         for (int w = w_b; w < w_e; ++w) {

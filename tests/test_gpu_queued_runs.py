@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from digital_twin_brain_b200 import Network, _lib, synthetic
-from digital_twin_brain_b200._lib import DTB_DEVICE
+from digital_twin_brain_b200._lib import DTB_DEVICE, FIELD_STEP, TUNE_PULL_METHOD
 from digital_twin_brain_b200.network import MODES
 
 pytestmark = pytest.mark.gpu
@@ -95,3 +95,34 @@ def test_captured_run_outlives_new_statistics_tables(N):
         np.testing.assert_array_equal(out[2].cpu().numpy().view(np.uint32),
                                       b.run(7, noise_rate=0.3, isolated=True, mode="push")[2])
     assert held[-1] - held[-2] <= 4096     # a few small tables a time
+
+
+@pytest.mark.parametrize("mode,method", [("push", 0), ("pull", 0), ("pull", 1), ("pull", 4)])
+def test_rows_start_with_their_run(mode, method, tmp_path):
+    """Row 0 belongs to the run's first step after everything that moves the clock: single steps, forced
+    steps, kernel timing, a step count set from outside, a checkpoint, a run of the small loop."""
+    spec = synthetic.single_block(20000, 20, gen_seed=1)
+    net = Network.from_spec(spec, device=0)
+    net.set_tuning(TUNE_PULL_METHOD, method)
+
+    def expected(step, n):      # the noise of each step, from a network that takes them one by one
+        ref = Network.from_spec(spec, device=0)
+        ref.set(FIELD_STEP, step)
+        return np.concatenate([ref.run(1, noise_rate=0.05, isolated=True, mode="push")[2] for _ in range(n)])
+
+    def check(n):
+        step = int(net.get(FIELD_STEP))
+        np.testing.assert_array_equal(net.run(n, noise_rate=0.05, isolated=True, mode=mode)[2], expected(step, n))
+    check(3)
+    net.run(1, noise_rate=0.2, mode=mode, out=None)
+    check(2)
+    net.step_forced(None, None, noise_rate=0.1, isolated=True, mode=mode)
+    check(2)
+    net.time_kernels(4, noise_rate=0.1, isolated=True, mode=mode)
+    check(40)
+    net.set(FIELD_STEP, 777)
+    check(2)
+    net.save(str(tmp_path / "ck.bin"))
+    net.run(5, noise_rate=0.1, mode=mode)
+    net.load(str(tmp_path / "ck.bin"))
+    check(35)
