@@ -1046,10 +1046,18 @@ static int ensure_slots(dtb_block* b)
     if (s.slots) return DTB_OK;
     uint32_t* cnt = nullptr; uint4* sl = nullptr;
     RET(dalloc(b, &cnt, (size_t)std::max<int64_t>(b->N, 1)));
-    RET(dalloc(b, &sl, (size_t)std::max<int64_t>(b->N, 1) * kSlotCap));
+    // 192 bytes a neuron, or 128 where the device has no more room (rows past it are gathered whole)
+    uint32_t cap = kSlotCap;
+    int rc = dalloc(b, &sl, (size_t)std::max<int64_t>(b->N, 1) * cap);
+    if (rc == DTB_ERR_NOMEM) {
+        cap = kSlotCapMin;
+        rc = dalloc(b, &sl, (size_t)std::max<int64_t>(b->N, 1) * cap);
+    }
+    if (rc != DTB_OK) { dfree(b, cnt); return rc; }
     CK(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (size_t)std::max<int64_t>(b->N, 1), b->stream));
     s.slot_cnt = cnt;
     s.slots = sl;
+    s.slot_cap = cap;
     drop_graphs(b);
     return DTB_OK;
 }

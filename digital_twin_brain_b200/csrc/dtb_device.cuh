@@ -19,7 +19,8 @@ namespace dtb {
 constexpr uint32_t kKindBit = 0x80000000u;
 constexpr uint32_t kIndexMask = 0x7fffffffu;
 constexpr int kWarpNeurons = 128;      // neurons owned by one warp in the step kernels
-constexpr uint32_t kSlotCap = 12;      // ordered-push contributions kept per neuron and step (even)
+constexpr uint32_t kSlotCap = 12;      // ordered-push contributions kept per neuron and step (even),
+constexpr uint32_t kSlotCapMin = 8;    // or these when memory is short
 constexpr int kGatherRows = 1;         // k_step gathers whole pull rows
 constexpr int kGatherSlots = 2;        // k_step sums its ordered-push slots
 constexpr int kGatherMasks = 3;        // k_step sums the pull entries its position masks mark
@@ -130,7 +131,8 @@ struct DevState {
     const uint16_t* qpos;       // [S] position of every push entry inside its pull row (nullable)
     // ordered push (bit-exact pull order at push cost): pending contributions per neuron
     uint32_t* slot_cnt;         // [N] contributions written since the neuron last consumed them
-    uint4* slots;               // [kSlotCap / 2][N][2] {pull-row position | kind bit, 0, w.x bits, w.y bits}
+    uint32_t slot_cap;          // records kept per neuron: kSlotCap or kSlotCapMin
+    uint4* slots;               // [slot_cap / 2][N][2] {pull-row position | kind bit, 0, w.x bits, w.y bits}
     uint32_t* pmask;            // [N][2][kMaskWords] pull-row positions that fired (excitatory, inhibitory)
     // binned push: the scatter appends every synaptic event {neuron within bin | kind << 15, w} to the bin of
     // its postsynaptic neuron; the next update folds each bin into its chunk in shared memory

@@ -1018,9 +1018,9 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
                     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
                     const uint32_t c = cnt[j];
                     if (c && c <= 4u) sum = slot_sum_few(c, s0[j], s1[j], s2[j - h], s3[j - h]);
-                    else if (c && c <= kSlotCap) sum = slot_sum_many(s.slots, s.N, n, c);
+                    else if (c && c <= s.slot_cap) sum = slot_sum_many(s.slots, s.N, n, c);
                     // overflowing rows: the warp gathers them whole, in row order
-                    unsigned m = __ballot_sync(0xffffffffu, c > kSlotCap);
+                    unsigned m = __ballot_sync(0xffffffffu, c > s.slot_cap);
                     while (m) {
                         const int l = __ffs(m) - 1;
                         m &= m - 1;
@@ -1607,7 +1607,7 @@ __global__ void __launch_bounds__(kScatterThreads, MINB) k_scatter(DevState s, i
                     }
 #pragma unroll
                     for (int u = 0; u < kScatterUnroll; ++u)
-                        if (k[u] < kSlotCap)
+                        if (k[u] < s.slot_cap)
                             __stcg(s.slots + slot_at(s.N, c[u] & kIndexMask, k[u]),
                                    make_uint4(ppos[u] | (c[u] & kKindBit), 0u, __float_as_uint(w[u].x), __float_as_uint(w[u].y)));
                 } else {

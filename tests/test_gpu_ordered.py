@@ -130,3 +130,32 @@ def test_masks_refused_beyond_128_inputs():
     with pytest.raises(DtbError):
         net.set_tuning(TUNE_PULL_METHOD, MASKS)
     net.run(20, noise_rate=0.02, mode="pull")      # auto: slots (in-degree 200 > 128)
+
+
+def test_slots_with_little_memory_left():
+    """12 records a neuron do not fit, 8 do: the ordered push runs with these, its results are the row
+    gather's (neurons with 9 to 12 contributions are gathered whole)."""
+    import torch
+    N = 2_000_000
+    spec = synthetic.single_block(N, 60, name="n2m_slots")
+    a, b = (Network.from_spec(spec, device=0) for _ in range(2))
+    a.set_tuning(TUNE_PULL_METHOD, ROWS)
+    b.set_tuning(TUNE_PULL_METHOD, SLOTS)
+    ref = [a.run(n, noise_rate=0.1, mode="pull") for n in (3, 9)]
+    want = _state(a)
+    a.close()
+    held = b.info().device_bytes
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    filler = torch.empty(free - (340 << 20), dtype=torch.uint8, device="cuda")    # 400 MB are wanted, 272 do
+    try:
+        got = [b.run(n, noise_rate=0.1, mode="pull") for n in (3, 9)]
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert b.info().device_bytes - held == N * (4 + 8 * 16)
+    for x, y in zip(ref, got):
+        for u, v in zip(x, y):
+            np.testing.assert_array_equal(u, v)
+    for x, y in zip(want, _state(b)):
+        np.testing.assert_array_equal(x, y)
