@@ -1435,20 +1435,28 @@ static BoldScalars<T> bold_scalars(const dtb_bold* m)
     return c;
 }
 
-static BoldConst bold_const(double eps, double ts, double tf, double t0, double alpha, double E0, double dt)
+// The constants of a float64 window; true: the fast form of its steps holds for them.
+static bool bold_const(const dtb_bold* m, BoldConst& c)
 {
-    BoldConst c;
-    c.eps = eps; c.r_ts = 1.0 / ts; c.r_tf = 1.0 / tf; c.r_t0 = 1.0 / t0; c.r_E0 = 1.0 / E0; c.dt = dt;
-    c.base = 1.0 - E0;
-    c.exv = 1.0 / alpha;
+    c.eps = m->eps; c.ts = m->ts; c.tf = m->tf; c.t0 = m->t0; c.E0 = m->E0; c.dt = m->dt;
+    c.base = 1.0 - m->E0;
+    c.exv = 1.0 / m->alpha;
+    c.exq = c.exv - 1.0;
     c.l_hi = c.l_lo = 0.0;
-    c.fast = (c.exv == 5.0 && c.base > 0.0 && c.base < 1.0) ? 1 : 0;
-    if (c.fast) {
+    bool fast = c.exv == 5.0 && c.base > 0.0 && c.base < 1.0;
+    const double y[4] = {c.ts, c.tf, c.t0, c.E0};
+    BoldRecip* r[4] = {&c.r_ts, &c.r_tf, &c.r_t0, &c.r_E0};
+    for (int i = 0; i < 4; ++i) {
+        r[i]->hi = 1.0 / y[i];
+        r[i]->lo = std::fma(-r[i]->hi, y[i], 1.0) / y[i];
+        fast = fast && std::fabs(y[i]) > 1e-6 && std::fabs(y[i]) < 1e6;   // neither part near the range's ends
+    }
+    if (fast) {
         const long double l = logl((long double)c.base);
         c.l_hi = (double)l;
         c.l_lo = (double)(l - (long double)c.l_hi);
     }
-    return c;
+    return fast;
 }
 
 // ------------------------------------------------------------ C ABI
@@ -2974,11 +2982,13 @@ int dtb_bold_run_steps(dtb_bold* m, const void* u, int n_steps, double u_floor, 
         k_bold_run_steps<float><<<gr, 128, 0, m->stream>>>(m->R, (const float*)du, n_steps, (float)u_floor,
                                                            (float*)m->s, (float*)m->q, (float*)m->v, (float*)m->f,
                                                            (float*)dout, bold_scalars<float>(m));
-    else
-        k_bold_run_steps_f64<<<grid_for(m->R, kBoldThreads), kBoldThreads, 0, m->stream>>>(
+    else {
+        BoldConst c;
+        auto* k = bold_const(m, c) ? k_bold_run_steps_f64<true> : k_bold_run_steps_f64<false>;
+        k<<<grid_for(m->R, kBoldThreads), kBoldThreads, 0, m->stream>>>(
             m->R, (const double*)du, n_steps, u_floor, (double*)m->s, (double*)m->q, (double*)m->v, (double*)m->f,
-            (double*)dout, bold_const(m->eps, m->ts, m->tf, m->t0, m->alpha, m->E0, m->dt), 7.0 * m->E0,
-            2.0 * m->E0 - 0.2, m->V0);
+            (double*)dout, c, 7.0 * m->E0, 2.0 * m->E0 - 0.2, m->V0);
+    }
     CK(cudaGetLastError());
     if (where == DTB_HOST) {
         CK(cudaMemcpyAsync(out, m->tmp_o, bytes, cudaMemcpyDeviceToHost, m->stream));

@@ -77,13 +77,13 @@ struct Ctl {
 };
 static_assert(sizeof(Ctl) == 64, "Ctl layout");
 
-// Constants of the float64 BOLD step (bold_model_pytorch.py:43-78): reciprocals of the time
-// constants and of E_0, and ln(1 - E_0) in two parts.
+// Constants of the float64 BOLD windows (bold_model_pytorch.py:43-78).
+struct BoldRecip { double hi, lo; };   // 1 / y
 struct BoldConst {
-    double eps, r_ts, r_tf, r_t0, r_E0, dt;
+    double eps, ts, tf, t0, E0, dt;
+    BoldRecip r_ts, r_tf, r_t0, r_E0;
     double base, l_hi, l_lo;   // 1 - E_0 and its logarithm
-    double exv;                // 1 / alpha
-    int fast;                  // 1: 1 / alpha is 5 and 0 < base < 1 (the model's own constants)
+    double exq, exv;           // 1 / alpha - 1 and 1 / alpha
 };
 
 struct BoldDev {

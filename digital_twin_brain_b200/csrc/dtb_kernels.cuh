@@ -263,56 +263,6 @@ __device__ __forceinline__ float4 mask_sum(const DevState& s, int64_t n, uint4 e
 }
 
 // ------------------------------------------------------------ BOLD step
-// base^(1/f), the oxygen extraction's power (f > 0).  With base in (0, 1): exp(ln(base) / f), the
-// product's rounding error and the low part of the logarithm added back to first order, so the
-// result is as exact as pow's; where that could underflow, and for any other base, pow itself.
-__device__ __forceinline__ double bold_extraction(const BoldConst& c, double f)
-{
-    const double x = 1.0 / f;
-    const double y = x * c.l_hi;
-    if (c.fast && y > -700.0) {
-        const double lo = fma(x, c.l_lo, fma(x, c.l_hi, -y));
-        const double e = exp(y);
-        return fma(e, lo, e);
-    }
-    return pow(c.base, x);
-}
-
-// v^(1/alpha - 1) and v^(1/alpha): by products for alpha = 0.2 (powers 4 and 5), else by pow.
-__device__ __forceinline__ void bold_powers(const BoldConst& c, double v, double& pq, double& pv)
-{
-    if (c.fast) {
-        const double v2 = v * v;
-        pq = v2 * v2;
-        pv = pq * v;
-    } else {
-        pq = pow(v, c.exv - 1.0);
-        pv = pow(v, c.exv);
-    }
-}
-
-// models/bold_model_pytorch.py:43-78 in float64 (q before v before f_in before s, f_in clamped
-// at 0) for windows of steps.  Three pow calls and six divisions made a step fp64-issue bound; with the products, one
-// exp and the reciprocals it has one division.
-__device__ __forceinline__ void bold_qv(const BoldConst& c, double f, double ext, double& q, double& v)
-{
-    double pq, pv;
-    bold_powers(c, v, pq, pv);
-    const double part = f > 0.0 ? 1.0 - ext : 1.0;
-    const double dq = ((f * part) * c.r_E0 - q * pq) * c.r_t0;
-    const double dv = (f - pv) * c.r_t0;
-    q = fma(dq, c.dt, q);
-    v = fma(dv, c.dt, v);
-}
-
-__device__ __forceinline__ void bold_fs(const BoldConst& c, double eu, double& f, double& s)
-{
-    const double ds = (eu - s * c.r_ts) - (f - 1.0) * c.r_tf;
-    f = fma(s, c.dt, f);
-    f = f > 0.0 ? f : 0.0;
-    s = fma(ds, c.dt, s);
-}
-
 // One step of region r with input u, for networks with BOLD attached: the reference's own operations
 // (pow, divisions), so that a bit-exact run's signal keeps its last bit; it runs beside the scatter.
 __device__ __forceinline__ void bold_region_step(const BoldDev& b, int r, double u)
@@ -2046,17 +1996,93 @@ __global__ void k_bold_run_steps(int64_t R, const T* __restrict__ u, int n_steps
     out[i] = ((c.k7 * (one - qi) + (one - qi / vi) * (T)2) + c.k2 * (one - vi)) * c.V0;
 }
 
-// The same in float64 (the hemodynamics of a forecast window: thousands of steps of a few
-// thousand regions, less than one warp per scheduler).  A region's (f_in, s) chain is short and
-// does not read q or v, so it runs kBoldAhead steps ahead and the steps' exponentials, which are
-// most of the work, are independent of each other.  One warp per CTA spreads the warps over all SMs.
-// 10,800 regions x 8,000 steps: 14.26 -> 2.02 ms (with the products and reciprocals of bold_qv).
+// The same in float64 (the hemodynamics of a forecast window: thousands of steps of a few thousand
+// regions, less than one warp per scheduler, so the latency of a step's dependent operations is the
+// time).  The (f_in, s) chain is short and does not read q or v, so it runs kBoldAhead steps ahead and
+// the steps' oxygen extractions, which are most of the work, are independent of each other.  One warp
+// per CTA spreads the warps over all SMs.
+// FAST (1 / alpha = 5, 0 < 1 - E_0 < 1): the powers and divisions, which the fp64 unit could not
+// overlap, by shorter operations that are no less exact, in the same order otherwise (largest / rms
+// error in ulp against quad precision, 262,144 values; before -> here):
+//   x / y with y fixed as x (hi + lo), hi + lo = 1 / y to twice the precision (Brisebarre, Muller and
+//   Raina, "Accelerating correctly rounded floating-point division when the divisor is known in
+//   advance", IEEE Trans. Computers 53, 2004): the same bits;
+//   v^4 and v^5 as products with their rounding errors carried along: 1.26 / 0.40 -> 0.50 / 0.29;
+//   base^(1/f) as exp of the product with ln(base) in two parts, whose rounding error is added back:
+//   1.24 / 0.38 -> 1.24 / 0.39 (and half an ulp of 1 - base^(1/f), four times as large, comes on top).
+// These do not hold for infinities and NaN: a group of steps that ends in one is taken again with the
+// plain operations.
+// 10,800 regions x 8,000 steps: 14.26 -> 2.17 ms (the plain operations in this order 13, with pow for the
+// extraction alone 4.9).  f_in and s have the bits of as many steps of k_bold_run, q and v to a few ulp.
+// Signal against the same steps in 80-bit arithmetic 3.2e-14 before and here; against torch in 64 bits,
+// whose pow rounds as the plain operations do, 7.5e-16 -> 8.5e-16.
 constexpr int kBoldAhead = 4;
 constexpr int kBoldThreads = 32;
 
+template <bool FAST>
+__device__ __forceinline__ double bold_div(double x, double y, const BoldRecip& r)
+{
+    return FAST ? fma(x, r.hi, x * r.lo) : x / y;
+}
+
+// base^(1/f), f > 0
+template <bool FAST>
+__device__ __forceinline__ double bold_extraction(const BoldConst& c, double f)
+{
+    const double x = 1.0 / f;
+    if (FAST) {
+        const double y = x * c.l_hi;
+        if (y > -700.0) {   // (exp neither underflows nor loses bits)
+            const double e = exp(y);
+            return fma(e, fma(x, c.l_lo, fma(x, c.l_hi, -y)), e);
+        }
+    }
+    return pow(c.base, x);
+}
+
+template <bool FAST>
+__device__ __forceinline__ void bold_fs(const BoldConst& c, double eu, double& f, double& s)
+{
+    const double ds = (eu - bold_div<FAST>(s, c.ts, c.r_ts)) - bold_div<FAST>(f - 1.0, c.tf, c.r_tf);
+    f = f + s * c.dt;
+    f = f > 0.0 ? f : 0.0;
+    s = s + ds * c.dt;
+}
+
+template <bool FAST>
+__device__ __forceinline__ void bold_qv(const BoldConst& c, double f, double ext, double& q, double& v)
+{
+    double pq, pv;
+    if (FAST) {
+        const double v2 = v * v, e2 = fma(v, v, -v2);
+        const double v4 = v2 * v2, e4 = fma(2.0 * v2, e2, fma(v2, v2, -v4));
+        const double v5 = v4 * v, e5 = fma(e4, v, fma(v4, v, -v5));
+        pq = v4 + e4;
+        pv = v5 + e5;
+    } else {
+        pq = pow(v, c.exq);
+        pv = pow(v, c.exv);
+    }
+    const double part = f > 0.0 ? 1.0 - ext : 1.0;
+    const double dq = bold_div<FAST>(bold_div<FAST>(f * part, c.E0, c.r_E0) - q * pq, c.t0, c.r_t0);
+    const double dv = bold_div<FAST>(f - pv, c.t0, c.r_t0);
+    q = q + dq * c.dt;
+    v = v + dv * c.dt;
+}
+
+__device__ __noinline__ void bold_plain(const BoldConst& c, double eu, int n, double& f, double& s, double& q, double& v)
+{
+    for (int k = 0; k < n; ++k) {
+        bold_qv<false>(c, f, f > 0.0 ? bold_extraction<false>(c, f) : 0.0, q, v);
+        bold_fs<false>(c, eu, f, s);
+    }
+}
+
+template <bool FAST>
 __global__ void __launch_bounds__(kBoldThreads) k_bold_run_steps_f64(int64_t R, const double* __restrict__ u, int n_steps,
                                                                      double floor_u, double* s, double* q, double* v,
-                                                                     double* f, double* __restrict__ out, BoldConst c,
+                                                                     double* f, double* __restrict__ out,
+                                                                     const __grid_constant__ BoldConst c,
                                                                      double k7, double k2, double V0)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2066,20 +2092,23 @@ __global__ void __launch_bounds__(kBoldThreads) k_bold_run_steps_f64(int64_t R, 
     int k = 0;
     for (; k + kBoldAhead <= n_steps; k += kBoldAhead) {
         double fa[kBoldAhead], ext[kBoldAhead];
+        double f1 = fi, s1 = si, q1 = qi, v1 = vi;
 #pragma unroll
         for (int j = 0; j < kBoldAhead; ++j) {
-            fa[j] = fi;
-            bold_fs(c, eu, fi, si);
+            fa[j] = f1;
+            bold_fs<FAST>(c, eu, f1, s1);
         }
 #pragma unroll
-        for (int j = 0; j < kBoldAhead; ++j) ext[j] = fa[j] > 0.0 ? bold_extraction(c, fa[j]) : 0.0;
+        for (int j = 0; j < kBoldAhead; ++j) ext[j] = fa[j] > 0.0 ? bold_extraction<FAST>(c, fa[j]) : 0.0;
 #pragma unroll
-        for (int j = 0; j < kBoldAhead; ++j) bold_qv(c, fa[j], ext[j], qi, vi);
+        for (int j = 0; j < kBoldAhead; ++j) bold_qv<FAST>(c, fa[j], ext[j], q1, v1);
+        if (FAST && !isfinite((f1 + s1) + (q1 + v1))) {
+            bold_plain(c, eu, kBoldAhead, fi, si, qi, vi);
+        } else {
+            fi = f1; si = s1; qi = q1; vi = v1;
+        }
     }
-    for (; k < n_steps; ++k) {
-        bold_qv(c, fi, fi > 0.0 ? bold_extraction(c, fi) : 0.0, qi, vi);
-        bold_fs(c, eu, fi, si);
-    }
+    bold_plain(c, eu, n_steps - k, fi, si, qi, vi);
     s[i] = si; q[i] = qi; v[i] = vi; f[i] = fi;
     out[i] = ((k7 * (1.0 - qi) + (1.0 - qi / vi) * 2.0) + k2 * (1.0 - vi)) * V0;
 }

@@ -379,7 +379,10 @@ int dtb_bold_run(dtb_bold* m, const void* u, void* out, int where);
 /* n_steps x BOLD.run with a constant input u[r] (floored at u_floor, as
  * simulation/simulation.py:279 floors at 1e-5); out = the last step's
  * signal.  Integrates the hemodynamics of a window whose rate is forecast
- * instead of simulated. */
+ * instead of simulated.  In float64, s and f_in have the bits of n_steps calls
+ * of dtb_bold_run; with the model's own alpha = 0.2, q and v (and the signal)
+ * may differ by the rounding of v^4, v^5 and (1 - E_0)^(1/f_in), which are
+ * taken without pow there. */
 int dtb_bold_run_steps(dtb_bold* m, const void* u, int n_steps, double u_floor, void* out, int where);
 /* BOLD.state_update (bold_model_pytorch.py:34-41): w is [E][Rp][S] of the
  * model's dtype with E*Rp == R; s = w[..,0], q = max(w[..,1],1e-5),
