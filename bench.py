@@ -485,7 +485,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
             # whole job at N replicas: the events of all ranks over the slowest rank's time
             e2e_ms, ev_e2e = combine_over_ranks(1000.0 * t_e2e, float(ev_e2e), world, f"cuda:{dev}")
             t_e2e = e2e_ms / 1000.0
-            h2d = 16                                  # run parameters (base step, noise rate, isolated)
+            h2d = 8                                   # run parameters (noise rate, isolated)
             d2h = 2 * 4 * net.n_sub + 4               # spike sums + mean V per subblock + propagated count
             e2e = {"value": ev_e2e / t_e2e, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                    "steps": E, "ms_per_step": 1000.0 * t_e2e / E,

@@ -161,9 +161,12 @@ struct dtb_block {
     // pinned host staging
     void* pinned = nullptr;
     size_t pinned_bytes = 0;
-    // the run parameters queued last (set_run_params)
-    bool run_set = false, run_isolated = false, run_replayed = false;
-    float run_rate = 0.0f;
+    // run parameters on their way to the device (set_run_params)
+    static constexpr int kRunSlots = 256;
+    RunParams* h_run = nullptr;                       // pinned [kRunSlots]
+    cudaEvent_t run_copied[2] = {nullptr, nullptr};   // the copies of each half of the slots have been made
+    int run_streams[2] = {1, 1};                      // streams they were queued on
+    uint64_t run_next = 0;
     // auto mode
     int64_t launches = 0;
     uint64_t samples_from = 0;    // step at which sampling started
@@ -569,6 +572,8 @@ static void destroy_block(dtb_block* b)
     for (void* p : b->allocs) cudaFree(p);
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
     if (b->pinned) cudaFreeHost(b->pinned);
+    if (b->h_run) cudaFreeHost(b->h_run);
+    for (cudaEvent_t ev : b->run_copied) if (ev) cudaEventDestroy(ev);
     delete b;
 }
 
@@ -577,6 +582,7 @@ static int rebuild_groups(dtb_block* b, const int32_t* sub_to_region);
 static int finish_create(dtb_block* b)
 {
     RET(rebuild_groups(b, nullptr));
+    CK(cudaMallocHost((void**)&b->h_run, sizeof(RunParams) * dtb_block::kRunSlots));
     RET(ensure_stats(b, 256));
     CK(cudaStreamSynchronize(b->stream));
     return DTB_OK;
@@ -1207,20 +1213,34 @@ static int upload_steps(dtb_block* b)
     return DTB_OK;
 }
 
-// The noise rate and isolation of the steps queued behind it, where they differ from the last ones
-// queued.  In a CUDA graph of the caller's they always go along, and from then on everywhere: a replay
-// may have come in between.
+// The noise rate and isolation of the steps queued behind it.  Each copy has a pinned slot of its own
+// until it has been made, so that runs queued before it keep theirs; in a CUDA graph of the caller's
+// they are a kernel's arguments, which every replay takes again.
 static int set_run_params(dtb_block* b, float noise_rate, int isolated)
 {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (!b->run_replayed && (cudaStreamIsCapturing(b->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone))
-        b->run_replayed = true;
-    if (!b->run_replayed && b->run_set && b->run_rate == noise_rate && b->run_isolated == (isolated != 0)) return DTB_OK;
-    k_set_run<<<1, 1, 0, b->stream>>>(b->ds.ctl, noise_rate, isolated ? 1 : 0);
-    CK(cudaGetLastError());
-    b->run_set = true;
-    b->run_rate = noise_rate;
-    b->run_isolated = isolated != 0;
+    if (cudaStreamIsCapturing(b->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();   // (the legacy stream beside another one's capture)
+        k_set_run<<<1, 1, 0, b->stream>>>(b->ds.ctl, noise_rate, isolated ? 1 : 0);
+        CK(cudaGetLastError());
+        return DTB_OK;
+    }
+    // the slots by halves: the event behind the last copy of a half covers them all, unless the network
+    // changed streams in between
+    constexpr int kHalf = dtb_block::kRunSlots / 2;
+    const int i = (int)(b->run_next % dtb_block::kRunSlots), half = i / kHalf;
+    if (i % kHalf == 0) {
+        if (b->run_streams[half] > 1) CK(cudaDeviceSynchronize());
+        else if (b->run_copied[half]) CK(cudaEventSynchronize(b->run_copied[half]));
+        b->run_streams[half] = 1;
+    }
+    ++b->run_next;
+    b->h_run[i] = RunParams{noise_rate, isolated ? 1 : 0};
+    CK(cudaMemcpyAsync(&b->ds.ctl->noise_rate, b->h_run + i, sizeof(RunParams), cudaMemcpyHostToDevice, b->stream));
+    if (i % kHalf == kHalf - 1) {
+        if (!b->run_copied[half]) CK(cudaEventCreateWithFlags(&b->run_copied[half], cudaEventDisableTiming));
+        CK(cudaEventRecord(b->run_copied[half], b->stream));
+    }
     return DTB_OK;
 }
 
@@ -1994,6 +2014,8 @@ int dtb_block_set_stream(dtb_block* b, void* stream)
     DeviceGuard g(b->device);
     if (b->stream != (cudaStream_t)stream) {
         drop_graphs(b);
+        const int at = (int)(b->run_next % dtb_block::kRunSlots);   // copies of the half at hand are on both streams
+        if (at % (dtb_block::kRunSlots / 2) != 0) b->run_streams[at / (dtb_block::kRunSlots / 2)]++;
     }
     b->stream = (cudaStream_t)stream;
     return DTB_OK;

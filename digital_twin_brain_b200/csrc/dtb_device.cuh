@@ -62,7 +62,7 @@ static_assert(sizeof(ParamClass) == 96, "ParamClass layout");
 struct Ctl {
     unsigned long long steps_done;   // number of completed updates (Philox step counter)
     unsigned long long run_base;     // steps_done at the start of the current run (stats row 0; DevState::last)
-    // run parameters (k_set_run)
+    // run parameters, written as one 8-byte copy (RunParams) or by k_set_run
     float noise_rate;                // >= 0: scalar rate; < 0: per-class rate
     int32_t isolated;                // block.run(isolated=...)
     float t;                         // block.t after the last update (float32 accumulation)
@@ -76,6 +76,12 @@ struct Ctl {
                                      // scatter that follows advances
 };
 static_assert(sizeof(Ctl) == 64, "Ctl layout");
+
+struct RunParams {
+    float noise_rate;
+    int32_t isolated;
+};
+static_assert(offsetof(Ctl, isolated) == offsetof(Ctl, noise_rate) + 4 && sizeof(RunParams) == 8, "RunParams layout");
 
 // Constants of the float64 BOLD windows (bold_model_pytorch.py:43-78).
 struct BoldRecip { double hi, lo; };   // 1 / y

@@ -413,9 +413,7 @@ __device__ __forceinline__ void deferred_stats(const DevState& s)
     }
 }
 
-// The parameters of the steps queued behind it: arguments by value, so that the calls and chunks
-// queued before these steps, and a replay of a caller's graph, each keep their own (a copy from one
-// host buffer would be read when the stream gets there).
+// The parameters of the steps behind it in a caller's CUDA graph.
 __global__ void k_set_run(Ctl* ctl, float noise_rate, int32_t isolated)
 {
     ctl->noise_rate = noise_rate;

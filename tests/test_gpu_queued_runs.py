@@ -126,3 +126,25 @@ def test_rows_start_with_their_run(mode, method, tmp_path):
     net.run(5, noise_rate=0.1, mode=mode)
     net.load(str(tmp_path / "ck.bin"))
     check(35)
+
+
+def test_many_queued_runs_on_changing_streams():
+    """More queued runs than parameter slots, on streams that take turns: each keeps its noise rate."""
+    spec = synthetic.single_block(20000, 4, gen_seed=1)
+    a, b = (Network.from_spec(spec, device=0) for _ in range(2))
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    rates = np.random.default_rng(0).uniform(0.0, 0.3, 700)
+    counts = torch.zeros((len(rates),), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for k, rate in enumerate(rates):
+        if k % 170 == 0:
+            other, side = streams[k // 170 % 2], streams[(k // 170 + 1) % 2]
+            side.wait_stream(other)                      # the runs follow each other
+            a.set_stream(side)
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(4_000_000)             # about 2 ms
+        _lib.call("dtb_block_run", a._h, 1, float(rate), 1, MODES["push"], None, None,
+                  ctypes.c_void_p(counts[k:].data_ptr()), DTB_DEVICE)
+    torch.cuda.synchronize()
+    want = np.concatenate([b.run(1, noise_rate=float(r), isolated=True, mode="push")[2] for r in rates])
+    np.testing.assert_array_equal(counts.cpu().numpy().view(np.uint32), want)
