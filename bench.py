@@ -46,10 +46,11 @@ sys.path.insert(0, ROOT)
 METRIC = "synaptic events/s & sim-s/wall-s at 2B syn; DA window time surrogate vs plain"
 UNIT = "events/s"
 # DRAM traffic per unit processed, from ncu captures (dram__bytes_read.sum + dram__bytes_write.sum)
-# of single launches: the atomic push scatter per synaptic event and the staged update per neuron.
+# at the whole-brain size (mean of 79 launches each): the atomic push scatter per synaptic event and
+# the staged update per neuron.
 # The line's roofline.traffic scales these to the launch it reports and says so.
-SCATTER_DRAM_BYTES_PER_EVENT = (943.26e6 + 360.44e6) / 23462598
-UPDATE_DRAM_BYTES_PER_NEURON = (595.12e6 + 418.77e6) / 23448955
+SCATTER_DRAM_BYTES_PER_EVENT = (1116.44e6 + 364.09e6) / 23568679
+UPDATE_DRAM_BYTES_PER_NEURON = (564.20e6 + 414.53e6) / 23448955
 
 
 def parse():
@@ -303,21 +304,33 @@ def roofline_of(spec, kt, mode, push_method, pull_method, peaks):
     return roofline, step
 
 
-def atomic_probe(dev, N, evs, window):
-    """float2 atomics per second on this GPU into J-sized targets (bench-only helper library)."""
+def scatter_probe(dev, N, ops, window, far, what=0):
+    """Milliseconds of `ops` scattered accesses into the J of N neurons (bench-only helper library):
+    float2 reductions (what 0), the same with the sectors prefetched into L2 (1), or ordered-push
+    records (2); a fraction `far` of the targets anywhere, the others inside a window that moves."""
     import ctypes
     from digital_twin_brain_b200 import build as B
     try:
-        L = ctypes.CDLL(B.build_probe())
-        fn = L.dtb_bench_atomic_rate
-        fn.argtypes = [ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.POINTER(ctypes.c_float)]
+        fn = ctypes.CDLL(B.build_probe()).dtb_bench_scatter_rate
+        fn.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.c_int,
+                       ctypes.POINTER(ctypes.c_float)]
         fn.restype = ctypes.c_int
         ms = ctypes.c_float()
-        if fn(dev, int(N), int(max(evs, 1)), int(max(1, window)), ctypes.byref(ms)) != 0:
+        if fn(dev, int(what), int(N), int(max(ops, 1)), int(min(N, max(1, window))), round(1000 * far), ctypes.byref(ms)) != 0:
             return None
         return ms.value
     except Exception:
         return None
+
+
+def print_scatter_rates(dev=0):
+    """The rates that the comments on the scatter quote: python -c "import bench; bench.print_scatter_rates()"."""
+    for N, window, far, label in ((1_000_000, 1_000_000, 0.0, "J in L2 (1e6 neurons), anywhere"),
+                                  (23_400_000, 260_000, 0.0, "whole-brain J, inside the region"),
+                                  (23_400_000, 260_000, 0.2, "whole-brain J, 80 % inside the region"),
+                                  (23_400_000, 260_000, 1.0, "whole-brain J, anywhere")):
+        r = [23_400_000 / scatter_probe(dev, N, 23_400_000, window, far, what) / 1e6 for what in range(3)]
+        print(f"{label}: float2 reductions {r[0]:.0f} G/s, prefetched {r[1]:.0f} G/s, claim + 16-byte store {r[2]:.0f} G/s")
 
 
 def mlp_measure(dev, peaks) -> dict:
@@ -501,19 +514,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
         pass
     roofline, step_roofline = roofline_of(spec, kt, mode, push_method, pull_method, peaks)
 
-    # the atomic push scatter's own ceiling: float2 atomics per second on this GPU, measured live with
-    # the same count into J-sized targets, destinations inside region-sized windows
-    atomic = None
     evs = kt["events_per_step"]
-    if mode == "push" and push_method != 2 and kt["propagate_ms"] > 0 and args.config != "profile_case":
-        probe_ms = atomic_probe(dev, spec.N, evs, spec.N // spec.R)
-        if probe_ms:
-            peak_ops = evs / (probe_ms * 1e-3) / 1e9
-            got_ops = evs / (kt["propagate_ms"] * 1e-3) / 1e9
-            atomic = {"bound": "l2_atomics", "achieved": got_ops, "peak": peak_ops, "unit": "G float2 atomics/s",
-                      "frac": got_ops / peak_ops, "kernel": "scatter",
-                      "probe": f"dtb_bench_atomic_rate(N={spec.N}, ops={int(evs)}, window={spec.N // spec.R})"}
-
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline and args.config in ("whole_brain",):
         r = cpu_sample(scale=1 / 64, noise=args.noise, seconds=15.0, max_steps=10_000)
@@ -543,7 +544,6 @@ def run_ours(args, rank: int, world: int, local_rank: int):
                 "kernel_ms": kt, "tune": tune, "build_s": t_build, "device_gb": info.device_bytes / 1e9,
                 "gpu_launches": int(launches),
                 "roofline": roofline,
-                "atomic_roofline": atomic,
                 "step_roofline": step_roofline,
                 "e2e": e2e,
                 "clocks": clk.summary()}

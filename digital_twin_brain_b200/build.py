@@ -16,7 +16,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 LIB = os.path.join(PKG, "libdtb.so")
-# bench.py's measurement helper (float2 atomic rate), kept out of libdtb.so
+# bench.py's measurement helper (rates of scattered reductions), kept out of libdtb.so
 PROBE_LIB = os.path.join(PKG, "libdtb_bench_probe.so")
 PROBE_SOURCES = ["bench_probe.cu"]
 
@@ -63,7 +63,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 def build_probe(force: bool = False) -> str:
-    """libdtb_bench_probe.so: the float2 atomic-rate probe bench.py reports beside the push scatter."""
+    """libdtb_bench_probe.so: the rates of scattered reductions that bench.print_scatter_rates prints."""
     srcs = [os.path.join(CSRC, f) for f in PROBE_SOURCES]
     if not force and os.path.exists(PROBE_LIB) and all(os.path.getmtime(f) <= os.path.getmtime(PROBE_LIB)
                                                         for f in srcs + [__file__]):

@@ -881,10 +881,13 @@ static int launch_gather_only(dtb_block* b, const DevState& s, int gather = kGat
     return DTB_OK;
 }
 
-// Bitmask words per warp: the caller's, or enough warps for every SM (a step's few firing rows
-// should not queue behind each other) and at most four words, past which a warp's rows serialise.
-// Measured, N = 31,013: 1 / 4 / 32 words 9.0 / 10.8 / 16.3 us; 1e6: 25.2 / 19.9 / 27.2; 1.2e7:
-// 226 / 196 / 243 (the row-list kernel).
+// Bitmask words per warp: the caller's, or enough warps for every SM (a step's few firing rows should
+// not queue behind each other; with one word a warp has one row a round, and many warps instead) and
+// at most four words, past which a warp's rows serialise.  us a push step at p = 0.01, 1 / 2 / 4 / 8 /
+// 32 words: N = 31,013 11.3 / 11.3 / 11.6 / 12.0 / 15.3; 1e5 9.6 / 9.8 / 10.0 / 10.6 / 16.1; 2.5e5
+// 15.1 / 14.2 / 15.6 / 17.9 / 22.0; 4e5 15.4 / 14.5 / 14.5 / 15.2 / 20.9; 1e6 26.2 / 23.1 / 22.3 / 22.5
+// / 38.2; 3.1e6 69 / 59 / 55 / 56 / 64; 1.2e7 300 / 272 / 268 / 268 / 305; 2.3e7 606 / 547 / 536 / 540 /
+// 611.  At p = 0.002 eight words are 1 to 5 % ahead from 1e6 on, at 0.05 two words 1 to 2 %.
 static int words_by_size(const dtb_block* b)
 {
     int w = 1;
@@ -897,8 +900,9 @@ static int scatter_words(const dtb_block* b)
     return b->scatter_wpw > 0 ? b->scatter_wpw : words_by_size(b);
 }
 
-// Prefetched targets pay once J no longer fits L2 (1.2e7 neurons, 195 MB of J: scatter 195 -> 180 us,
-// step 279 -> 267); while it does they only cost (1e6: 17.0 -> 21.3 us).
+// Prefetched targets pay once J no longer fits L2, while it does they only cost.  us a push step, not
+// prefetched / prefetched, p = 0.01: 1e6 neurons (16 MB of J) 22.3 / 26.4, 3.1e6 (50 MB) 55 / 65,
+// 1.2e7 (196 MB) 280 / 268, 2.3e7 (375 MB) 575 / 536.
 static int scatter_form(const dtb_block* b)
 {
     return (16 * b->N > ((int64_t)126 << 20) ? 1 : 0) ^ b->scatter_variant;

@@ -1463,9 +1463,11 @@ __global__ void __launch_bounds__(kStepThreads, MINB) k_step(DevState s, int til
 // weight pair to the pending J with one float2 reduction.  No row lists, scans or searches: a row
 // costs its loads and four shuffles, and a small `wpw` spreads the few rows of a step over enough
 // warps that their dependent reads (word, bounds, synapses) overlap.  The synapse stream is read
-// evict-first so that it does not push J out of L2.  Rate: 180 G reductions/s while J is in L2;
-// J lines that have to come from memory make it 112 G/s (targets of a region, 384 MB of J) and
-// 31 G/s (targets anywhere).
+// evict-first so that it does not push J out of L2.  What bounds it: while J is in L2, the chain of
+// dependent reads (float2 reductions alone make 170 G/s there); past that the J sectors, which come
+// from memory and go back (2.36e7 events into 375 MB of J: 63 bytes of DRAM traffic an event, 1.48 GB
+// in 0.36 ms = 4.1 TB/s, 63 % of a copy's rate; reductions alone to targets of the same spread, a
+// fifth of them anywhere, 43 to 47 G/s, the kernel 65 G/s).
 constexpr int kScatterThreads = 256;
 constexpr int kScatterMaxWords = 32;
 constexpr int kScatterRows = 2;                             // rows walked together
