@@ -1407,7 +1407,7 @@ static int run_small(dtb_block* b, int ctas, int n, float noise_rate, int isolat
     a.n_steps = n;
     a.tiles_per_cta = (nt + ctas - 1) / ctas;
     a.cap = (uint32_t)small_cap(a.tiles_per_cta);
-    a.tile_magic = (65536u + (uint32_t)a.tiles_per_cta - 1u) / (uint32_t)a.tiles_per_cta;   // exact for tile < 96 (tested)
+    a.tile_magic = small_magic(a.tiles_per_cta);
     a.isolated = isolated ? 1 : 0;
     a.noise_rate = noise_rate;
     a.write_v = b->ds.n_samples > 0 ? 1 : 0;

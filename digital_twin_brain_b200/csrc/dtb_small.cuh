@@ -51,6 +51,17 @@ inline int small_cap(int tiles)
 }
 static_assert((long long)kSmallTiles * kWarpNeurons * (kSmallCell + 12 * kSmallCapMin) + kSmallBits <= kSmallSmemMax, "shared memory");
 
+// tile / tiles_per_cta as a product and a shift, for every tile of the largest network
+constexpr uint32_t small_magic(int tiles_per_cta) { return (65536u + (uint32_t)tiles_per_cta - 1u) / (uint32_t)tiles_per_cta; }
+constexpr bool small_magic_exact()
+{
+    for (uint32_t c = 1; c <= (uint32_t)kSmallTiles; ++c)
+        for (uint32_t t = 0; t < (uint32_t)(kSmallTiles * kSmallClusterMax); ++t)
+            if ((t * small_magic((int)c)) >> 16 != t / c) return false;
+    return true;
+}
+static_assert(small_magic_exact(), "tile division");
+
 struct SmallArgs {
     int n_steps;
     int tiles_per_cta;

@@ -40,11 +40,11 @@ def test_ordered_push_matches_reference_golden(method):
 
 
 @pytest.mark.parametrize("method", [SLOTS, MASKS, STREAM], ids=["slots", "masks", "stream"])
-@pytest.mark.parametrize("rate,K", [(0.01, 100), (0.05, 120), (0.3, 60)],
-                         ids=["sparse", "overflowing_rows", "dense"])
+@pytest.mark.parametrize("rate,K", [(0.01, 100), (0.05, 120), (0.1, 100), (0.3, 60)],
+                         ids=["sparse", "few_overflowing_rows", "full_slots", "dense"])
 def test_ordered_push_equals_row_gather(rate, K, method):
-    """Slots: rows with more than 8 contributions per step fall back to the warp gather inside the same
-    kernel.  Masks: one bit per pull-row position (in-degree up to 128)."""
+    """Slots: rows with more than 12 contributions per step fall back to the warp gather inside the same
+    kernel (full_slots: 10 on average, so that many rows have 9 to 12 and as many just more).  Masks: one bit per pull-row position (in-degree up to 128)."""
     spec = synthetic.whole_brain(R=6, mean_size=700, sigma=0.5, K=K, gen_seed=3, name=f"wb6_K{K}")
     a = Network.from_spec(spec, device=0)
     b = Network.from_spec(spec, device=0)

@@ -201,11 +201,12 @@ def test_scatter_shapes_agree_with_pull_under_forcing(wpw, variant, reverse):
     np.testing.assert_allclose(a.get(FIELD_J), b.get(FIELD_J), rtol=1e-5, atol=1e-6)
 
 
-def test_chunked_and_graph_runs_are_identical():
-    spec = synthetic.single_block(5000, 50, name="n5k")
+@pytest.mark.parametrize("N", [20000, 5000], ids=["chunk_graphs", "cluster_loop"])
+def test_chunked_and_graph_runs_are_identical(N):
+    spec = synthetic.single_block(N, 50, name="n5k")
     a = Network.from_spec(spec, device=0)
     b = Network.from_spec(spec, device=0)
-    sa, ma, na = a.run(100, mode="pull")          # chunks of 32 through CUDA graphs
+    sa, ma, na = a.run(100, mode="pull")          # chunks of 32 through CUDA graphs, or launches of the loop
     rows = [b.run(1, mode="pull") for _ in range(100)]
     assert np.array_equal(sa, np.concatenate([r[0] for r in rows]))
     assert np.array_equal(ma, np.concatenate([r[1] for r in rows]))

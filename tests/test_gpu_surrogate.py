@@ -71,6 +71,27 @@ def test_shapes_match_oracle(inputs, hidden, B):
     assert np.abs(g.cpu().numpy() - g_ref).max() <= 1e-4 * np.abs(g_ref).max()
 
 
+@pytest.mark.parametrize("inputs", [14, 32])
+@pytest.mark.parametrize("B", [4736, 4737, 9472, 9473, 11521, 37889])
+def test_row_copies_match_oracle(inputs, B):
+    """The fused kernels at the row counts where a tile holds four, two or one copy of each row, whole
+    and partial last tiles, more tiles than SMs."""
+    rng = np.random.default_rng([B, inputs])
+    m = MLP(inputs, 256, seed=5, device=0)
+    x = rng.normal(0, 1, (B, inputs)).astype(np.float32)
+    t = rng.normal(0, 1, B).astype(np.float32)
+    y_ref, loss_ref, g_ref = mlp_oracle.forward_backward(m.params(), x, t, inputs, 256)
+    y = m.forward(torch.from_numpy(x)).cpu().numpy()
+    g, loss = m.gradient(torch.from_numpy(x), torch.from_numpy(t))
+    g = g.cpu().numpy()
+    # float32 sums of 256 terms (16 roundings of 2^-24 as a random walk, 1e-6) through two layers and,
+    # for the gradient, sums over the batch; a BF16 term lost from a split would be 2^-17 = 8e-6 or more
+    for part, ref in ((y, y_ref), (g, g_ref)):
+        assert np.linalg.norm(part - ref) <= 4e-6 * np.linalg.norm(ref)
+    assert np.abs(y - y_ref).max() <= 1e-5 * np.abs(y_ref).max()
+    assert abs(loss - loss_ref) <= 1e-5 * loss_ref
+
+
 @pytest.mark.parametrize("hidden", [256, 64])
 def test_failed_growth_leaves_other_owners_alone(hidden):
     """Activations that cannot grow: the call reports it, the network stays usable, and closing it
