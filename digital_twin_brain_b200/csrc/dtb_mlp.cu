@@ -478,8 +478,8 @@ __global__ void k_adam(int64_t n, float* w, const float* __restrict__ g, float* 
     v[i] = vi;
     w[i] = wi;
     const __nv_bfloat16 h = __float2bfloat16_rn(wi);
-    wb[i] = h;
     if (img) net_write_img(i, in, kx, h, img);
+    else wb[i] = h;
 }
 
 __global__ void k_to_bf16(int64_t n, const float* __restrict__ w, __nv_bfloat16* wb, __nv_bfloat16* img, int in, int kx)
@@ -487,8 +487,25 @@ __global__ void k_to_bf16(int64_t n, const float* __restrict__ w, __nv_bfloat16*
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const __nv_bfloat16 h = __float2bfloat16_rn(w[i]);
-    wb[i] = h;
     if (img) net_write_img(i, in, kx, h, img);
+    else wb[i] = h;
+}
+
+// A new network: zero moments and error flag, the compute copy of its weights, and zeros for the
+// padded inputs of W1's image.
+__global__ void k_init(int64_t n, const float* __restrict__ w, float* m, float* v, __nv_bfloat16* wb, __nv_bfloat16* img,
+                       int in, int kx, unsigned* err)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *err = 0u;
+    if (img && i < (int64_t)kNetH * (kx - in))
+        img[2 * kNetImgW2 + net_img(kNetH, (int)(i / (kx - in)), in + (int)(i % (kx - in)))] = __float2bfloat16_rn(0.0f);
+    if (i >= n) return;
+    m[i] = 0.0f;
+    v[i] = 0.0f;
+    const __nv_bfloat16 h = __float2bfloat16_rn(w[i]);
+    if (img) net_write_img(i, in, kx, h, img);
+    else wb[i] = h;
 }
 
 }  // namespace
@@ -502,8 +519,8 @@ struct dtb_mlp {
     int64_t o_W1, o_b1, o_W2, o_b2, o_W3, o_b3;
     void* tail = nullptr;          // the allocation of the operand images and the error flag
     float* w = nullptr;            // FP32 master [n_params]
-    __nv_bfloat16* wb = nullptr;   // BF16 compute copy
-    __nv_bfloat16* img = nullptr;  // fused kernels: W2, W2^T and W1 as operand images (null: layer by layer)
+    __nv_bfloat16* wb = nullptr;   // BF16 compute copy (layer by layer)
+    __nv_bfloat16* img = nullptr;  // fused kernels: W2, W2^T and W1 as operand images, then W3 (null: layer by layer)
     int kx = 0;                    // ... padded inputs
     float* g = nullptr;            // gradients, then the loss
     float* m = nullptr;            // Adam moments
@@ -637,7 +654,7 @@ int net_pass(dtb_mlp* p, const float* x, const float* target, int64_t B, float* 
     g.x = x; g.target = target;
     g.img2 = p->img; g.img2t = p->img + kNetImgW2; g.img1 = p->img + 2 * kNetImgW2;
     g.b1 = p->w + p->o_b1; g.b2 = p->w + p->o_b2; g.b3 = p->w + p->o_b3;
-    g.w3 = p->wb + p->o_W3;
+    g.w3 = p->img + kNetImgW3;
     g.y = y; g.err = p->err; g.wait = p->wait_limit;
     // the most copies of a row that still fit one CTA per SM in one wave
     const int D = cdiv(B, kNetRows / 4) <= kNetSMs ? 4 : (cdiv(B, kNetRows / 2) <= kNetSMs ? 2 : 1);
@@ -752,10 +769,10 @@ int dtb_mlp_create(int in_dim, int hidden, uint64_t seed, int device, dtb_mlp** 
     for (int64_t i = 0; i < hidden; ++i) w[(size_t)(p->o_W3 + i)] = (2.0f * uni() - 1.0f) * a2;
     const bool fused = hidden == kNetH && in_dim <= kNetMaxIn;
     const size_t f4 = sizeof(float) * (size_t)o;
-    const size_t fi = fused ? sizeof(__nv_bfloat16) * (size_t)(2 * kNetImgW2 + kNetH * kNetMaxIn) : 0;
+    const size_t fi = fused ? sizeof(__nv_bfloat16) * (size_t)kNetImg : 0;
     unsigned char* tail = nullptr;   // operand images, then the error flag
     cudaError_t e = cudaMalloc(&p->w, f4);
-    if (e == cudaSuccess) e = cudaMalloc(&p->wb, sizeof(__nv_bfloat16) * (size_t)o);
+    if (e == cudaSuccess && !fused) e = cudaMalloc(&p->wb, sizeof(__nv_bfloat16) * (size_t)o);
     if (e == cudaSuccess) e = cudaMalloc(&p->g, f4 + sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&p->m, f4);
     if (e == cudaSuccess) e = cudaMalloc(&p->v, f4);
@@ -768,10 +785,6 @@ int dtb_mlp_create(int in_dim, int hidden, uint64_t seed, int device, dtb_mlp** 
             p->kx = in_dim <= 16 ? 16 : 32;
             p->img = (__nv_bfloat16*)tail;
         }
-        // zero moments, error flag and the padded inputs' weights
-        e = cudaMemset(p->m, 0, f4);
-        if (e == cudaSuccess) e = cudaMemset(p->v, 0, f4);
-        if (e == cudaSuccess) e = cudaMemset(tail, 0, fi + sizeof(unsigned));
     }
     static std::atomic<uint64_t> ready{0};   // devices whose attributes are set
     if (e == cudaSuccess && fused && !((ready.load() >> (device & 63)) & 1)) {
@@ -784,8 +797,9 @@ int dtb_mlp_create(int in_dim, int hidden, uint64_t seed, int device, dtb_mlp** 
     }
     if (e == cudaSuccess) e = cudaMemcpy(p->w, w.data(), sizeof(float) * (size_t)o, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
-        k_to_bf16<<<cdiv(o, 256), 256>>>(o, p->w, p->wb, p->img, in_dim, p->kx);
-        e = cudaDeviceSynchronize();
+        k_init<<<cdiv(o, 256), 256>>>(o, p->w, p->m, p->v, p->wb, p->img, in_dim, p->kx, p->err);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaDeviceSynchronize();
     }
     if (prev >= 0) cudaSetDevice(prev);
     if (e != cudaSuccess) {

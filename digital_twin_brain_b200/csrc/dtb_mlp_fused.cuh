@@ -525,10 +525,14 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_grad(GradArgs g)
     }
 }
 
-// Where weight p of the flat order lies in the operand images (in inputs, hidden = 256).
+// Weight p of the flat order into the operand images (in inputs, hidden = 256) and W3 behind them.
+constexpr int kNetImgW3 = 2 * kNetImgW2 + kNetH * kNetMaxIn;        // elements: W2, W2^T, W1
+constexpr int kNetImg = kNetImgW3 + kNetH;
+
 __device__ __forceinline__ void net_write_img(int64_t p, int in, int kx, __nv_bfloat16 w, __nv_bfloat16* img)
 {
-    const int64_t o2 = (int64_t)kNetH * in + kNetH;
+    const int64_t o2 = (int64_t)kNetH * in + kNetH, o3 = o2 + kNetImgW2 + kNetH;
+    if (p >= o3 && p < o3 + kNetH) img[kNetImgW3 + (p - o3)] = w;
     if (p < (int64_t)kNetH * in) {
         img[2 * kNetImgW2 + net_img(kNetH, (int)(p / in), (int)(p % in))] = w;
     } else if (p >= o2 && p < o2 + kNetImgW2) {
