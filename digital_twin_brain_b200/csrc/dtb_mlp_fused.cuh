@@ -154,8 +154,8 @@ static_assert(kNetSmem <= 227 * 1024, "shared memory of one CTA");
 // spends 1 / D of the time on the elementwise work that bounds it (gradient of 4,096 rows 124 -> 87 us,
 // Adam step on 360 rows 92 -> 54 us against D = 1).
 // A thread whose wait is given up on stores nothing from then on, nor does any other after the next
-// barrier, where no further MMAs are issued either: y of the CTA's rows and the loss become NaN, and
-// the error flag keeps the weight gradients and Adam from using what was not computed.
+// barrier, where no further MMAs are issued either: y and dY of the CTA's rows and the loss become
+// NaN, and the error flag keeps Adam from using what was not computed.
 template <bool TRAIN, int D>
 __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
 {
@@ -346,6 +346,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     ok = __syncthreads_and(ok);
+    if (TRAIN && !ok && tid < kRows && live) g.dY[row] = nanf("");
     if (!ok) {   // a wait was given up on: flag it, and let copies and MMAs in flight land before shared memory and TMEM go
         if (tid == 0) {
             if (g.err) atomicOr(g.err, 1u);
@@ -483,9 +484,8 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_grad(GradArgs g)
             ++n_st;
         }
     }
-    const unsigned earlier = tid == 0 ? __ldcg(g.err) : 0u;   // a pass before gave up: there is nothing to add
     if (st > 0) ok = ok && mma_wait(mb, (uint32_t)((st - 1) & 1), g.wait);
-    ok = __syncthreads_and(ok && earlier == 0u);
+    ok = __syncthreads_and(ok);
     if (!ok && tid == 0) {   // a wait was given up on: nothing is added, and MMAs in flight end before TMEM goes
         atomicOr(g.err, 1u);
         atomicAdd(g.loss, nanf(""));

@@ -431,8 +431,8 @@ int dtb_mlp_gradient(dtb_mlp* m, const float* x, const float* target, int64_t B,
 /* one Adam step (beta 0.9 / 0.999, eps 1e-8) on that loss */
 int dtb_mlp_train_step(dtb_mlp* m, const float* x, const float* target, int64_t B, float lr, float* loss);
 /* Every wait of the tensor-core kernels is bounded.  A pass that gave one up returns NaN (y of its
- * rows, the loss), and until dtb_mlp_get_params has reported it (DTB_ERR_CUDA, once) gradients stay
- * zero with a NaN loss and Adam steps change no weights.  polls: the bound for hidden = 256 and at
+ * rows, the loss; a gradient beside a NaN loss is not one), and Adam steps change no weights from then
+ * on until dtb_mlp_get_params has reported it (DTB_ERR_CUDA, once).  polls: the bound for hidden = 256 and at
  * most 32 inputs (0: every wait is given up at once). */
 int dtb_mlp_set_wait_limit(dtb_mlp* m, uint32_t polls);
 int dtb_mlp_last_error(char* buf, size_t len);

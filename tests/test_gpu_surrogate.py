@@ -137,8 +137,7 @@ def test_given_up_waits_yield_no_results(B, limit):
     given_up = bool(lost.any()) or np.isnan(loss)
     if given_up:
         _lib.call("dtb_mlp_set_wait_limit", m._h, 1 << 22)
-        assert np.isnan(m.gradient(x, t)[1])            # not reported yet
-        m.train_step(x, t, 1e-2)
+        m.train_step(x, t, 1e-2)                        # not reported yet
         with pytest.raises(DtbError):
             m.params()
         np.testing.assert_array_equal(m.params(), w)    # reported once; the step changed nothing
