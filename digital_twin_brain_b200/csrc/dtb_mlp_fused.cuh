@@ -124,6 +124,10 @@ __device__ __forceinline__ void net_split8(const float* x, unsigned char* dst, i
             *reinterpret_cast<uint4*>(dst + i * term_bytes + d * dup_bytes) = make_uint4(t[i][0], t[i][1], t[i][2], t[i][3]);
 }
 
+// What was given up on lands before its shared memory and TMEM go (out of line: rarely run, and the
+// kernels' loops are long enough for the instruction cache to notice).
+__device__ __noinline__ void net_drain(uint32_t mbar, uint32_t parity) { mma_wait(mbar, parity, kNetDrain); }
+
 struct NetArgs {
     int in, kx;                            // inputs, padded K of layer 1
     int64_t B;
@@ -153,9 +157,9 @@ static_assert(kNetSmem <= 227 * 1024, "shared memory of one CTA");
 // the D quadrants share a row's columns, so that a batch too small to fill the GPU with 128-row tiles
 // spends 1 / D of the time on the elementwise work that bounds it (gradient of 4,096 rows 124 -> 87 us,
 // Adam step on 360 rows 92 -> 54 us against D = 1).
-// A thread whose wait is given up on stores nothing from then on, nor does any other after the next
-// barrier, where no further MMAs are issued either: y and dY of the CTA's rows and the loss become
-// NaN, and the error flag keeps Adam from using what was not computed.
+// Once a wait was given up on, in any thread: y and dY of the CTA's rows and the loss become NaN, and
+// the error flag keeps Adam from using what was not computed.  (Told to all at the barrier before the
+// output and at the end; at every chunk's barrier it cost the forward of 11,520 rows 0.3 us more.)
 template <bool TRAIN, int D>
 __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
 {
@@ -239,8 +243,8 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
                        D, kRows * 16);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        ok = __syncthreads_and(ok);
-        if (tid == 0 && ok) {
+        __syncthreads();
+        if (tid == 0 && ok) {   // (so that at most one commit is outstanding when a wait is given up)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int k8 = (q - q0) * (kNetChunk / 8);
             for (int s = 0; s < kNetChunk / 16; ++s)
@@ -345,16 +349,17 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(NetArgs g)
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    ok = __syncthreads_and(ok);
+    if (TRAIN) ok = __syncthreads_and(ok);
+    else __syncthreads();
     if (TRAIN && !ok && tid < kRows && live) g.dY[row] = nanf("");
     if (!ok) {   // a wait was given up on: flag it, and let copies and MMAs in flight land before shared memory and TMEM go
         if (tid == 0) {
             if (g.err) atomicOr(g.err, 1u);
             if (TRAIN) atomicAdd(g.loss, nanf(""));
-            mma_wait(b_w1, 0, kNetDrain);
-            mma_wait(b_w2, w2t ? 1u : 0u, kNetDrain);
-            if (l1) mma_wait(b_l1, 0, kNetDrain);
-            if (n_ch) mma_wait(b_ch, (uint32_t)((n_ch - 1) & 1), kNetDrain);
+            net_drain(b_w1, 0u);
+            net_drain(b_w2, w2t ? 1u : 0u);
+            if (l1) net_drain(b_l1, 0u);
+            if (n_ch) net_drain(b_ch, (uint32_t)((n_ch - 1) & 1));
         }
         __syncthreads();
     }
@@ -466,7 +471,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_grad(GradArgs g)
             net_split8(v, gsm + kGradOffX + (c * (g.kx / 8) + (f >> 3)) * 128 + (f & 7) * 16, kGradX);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        ok = __syncthreads_and(ok);
+        __syncthreads();
         if (tid == 0 && ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int s = 0; s < kGradStage / 16; ++s)
@@ -485,12 +490,12 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_grad(GradArgs g)
         }
     }
     if (st > 0) ok = ok && mma_wait(mb, (uint32_t)((st - 1) & 1), g.wait);
-    ok = __syncthreads_and(ok);
-    if (!ok && tid == 0) {   // a wait was given up on: nothing is added, and MMAs in flight end before TMEM goes
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok && lane == 0) {   // a wait was given up on: the warp adds nothing, the loss says so
         atomicOr(g.err, 1u);
         atomicAdd(g.loss, nanf(""));
-        if (n_st) mma_wait(mb, (uint32_t)((n_st - 1) & 1), kNetDrain);
     }
+    if (!ok && tid == 0 && n_st) net_drain(mb, (uint32_t)((n_st - 1) & 1));   // MMAs in flight end before TMEM goes
     if (st > 0 && ok) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // thread: output row 128 x + 32 (w % 4) + lane, 128 of the 256 columns
