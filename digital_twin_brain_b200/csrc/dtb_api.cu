@@ -903,10 +903,9 @@ static int scatter_words(const dtb_block* b)
 // Prefetched targets pay once J no longer fits L2, while it does they only cost.  us a push step, not
 // prefetched / prefetched, p = 0.01: 1e6 neurons (16 MB of J) 22.3 / 26.4, 3.1e6 (50 MB) 55 / 65,
 // 1.2e7 (196 MB) 280 / 268, 2.3e7 (375 MB) 575 / 536.
-static int scatter_form(const dtb_block* b)
-{
-    return (16 * b->N > ((int64_t)126 << 20) ? 1 : 0) ^ b->scatter_variant;
-}
+static int form_by_size(const dtb_block* b) { return 16 * b->N > ((int64_t)126 << 20) ? 1 : 0; }
+
+static int scatter_form(const dtb_block* b) { return form_by_size(b) ^ b->scatter_variant; }
 
 // how: kScatterJ (push), kScatterSlots / kScatterMasks (ordered push)
 static int launch_scatter(dtb_block* b, const DevState& s_in, int how = kScatterJ, bool defer = false, bool last = false)
@@ -2329,8 +2328,9 @@ int dtb_block_autotune(dtb_block* b, int n_steps, float noise_rate, float* repor
     if (b->has_push) {
         const int cand[6] = {1, 2, 4, 8, 16, 32};
         int best_sv = b->scatter_variant;
-        for (int sv = 0; sv < 2; ++sv)
+        for (int form = 0; form < 2; ++form)   // plain, then prefetched
             for (int w : cand) {
+                const int sv = form ^ form_by_size(b);
                 b->scatter_wpw = w;
                 b->scatter_variant = sv;
                 float o[4];
